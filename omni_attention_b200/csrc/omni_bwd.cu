@@ -48,8 +48,8 @@ struct BwdCfg {
 
 constexpr int kBwdComputeThreads = 256;
 constexpr int kBwdThreads = kBwdComputeThreads + 64;
-constexpr int kBwdIssuer = kBwdComputeThreads;         // thread that issues the MMAs
-constexpr int kBwdProducer = kBwdComputeThreads + 32;  // thread that issues the TMA loads
+constexpr int kBwdIssuerWarp = kBwdComputeThreads / 32;         // one elected lane issues the MMAs
+constexpr int kBwdProducerWarp = kBwdComputeThreads / 32 + 1;   // one elected lane issues the TMA loads
 
 
 template <bool BF16>
@@ -121,10 +121,11 @@ __device__ __forceinline__ void bwd_load_tile(uint32_t dst, const CUtensorMap* t
   for (int c = 0; c < BwdCfg<D>::kChunks; ++c) tma_load_2d(dst + c * BwdCfg<D>::kChunkBytes, tm, bar, c * 64, y);
 }
 
-// Every tcgen05.mma occupies the issuing thread for about as long as the tensor pipe needs for it, so
-// whatever else that thread executes per MMA is time with nothing queued: the descriptors are advanced
-// as 32-bit low words (the high word is one constant) and the accumulate flags are compile-time
-// constants wherever they can be.
+// The issuing thread runs ahead of the tensor pipe by about eight MMAs as long as it spends less time on
+// an MMA than the pipe does (64 cycles at 128x128x16): the thread is chosen with elect.sync (an MMA issued
+// under a branch on the lane number costs the thread 52 cycles, under an elected branch 17), the
+// descriptors are advanced as 32-bit low words (the high word is one constant) and the accumulate flags
+// are compile-time constants wherever they can be.
 constexpr uint32_t kBwdDescHi = umma_desc_hi_sw128(1024);
 
 // acc[128 x 128] = A[128 x D] * B[128 x D]^T, both tiles row-major with D contiguous (K-major).
@@ -369,7 +370,7 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   __syncthreads();   // the LSE / delta vectors are read by every compute thread
 
-  if (tid == kBwdProducer) {
+  if (warp == kBwdProducerWarp && elect_one()) {
     // =========================== TMA producer ====================================================
     if (n_vis > 0) {
       mbar_expect_tx(bar_kv, 2 * Cfg::kTileBytes);
@@ -389,7 +390,7 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       mbar_expect_tx(bar_do + 8 * stage, Cfg::kTileBytes);
       bwd_load_tile<D>(sdO + stage * Cfg::kTileBytes, &tmdO, bar_do + 8 * stage, y);
     }
-  } else if (tid == kBwdIssuer) {
+  } else if (warp == kBwdIssuerWarp && elect_one()) {
     // =========================== MMA issuer ======================================================
     for (int i = 0; i < n_vis; ++i) {
       const int stage = i & 1;
@@ -705,7 +706,7 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   const int n_vis = *n_vis_s;
 
-  if (tid == kBwdProducer) {
+  if (warp == kBwdProducerWarp && elect_one()) {
     // =========================== TMA producer ====================================================
     if (n_vis > 0) {
       mbar_expect_tx(bar_qdo, 2 * Cfg::kTileBytes);
@@ -723,7 +724,7 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_expect_tx(bar_v + 8 * vs, Cfg::kTileBytes);
       bwd_load_tile<D>(sV + vs * Cfg::kTileBytes, &tmV, bar_v + 8 * vs, y);
     }
-  } else if (tid == kBwdIssuer) {
+  } else if (warp == kBwdIssuerWarp && elect_one()) {
     // =========================== MMA issuer ======================================================
     auto issue_s = [&](int j) {    // S(j) = Q K(j)^T
       mbar_wait(bar_k + 8 * (j % 3), static_cast<uint32_t>((j / 3) & 1), abort_flag, p.f.status, 61);

@@ -22,6 +22,21 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// True in exactly one lane of the (converged) warp. A branch on it, unlike one on the lane number, tells
+// the compiler that a single thread is active, so that the operands tcgen05.mma and the bulk copies
+// want in uniform registers are moved there once instead of in a loop over the possibly active lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(pred));
+  return pred != 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------
