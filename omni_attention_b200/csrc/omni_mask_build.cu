@@ -17,10 +17,13 @@
 // dense rule. PARTIAL tiles are written bit-packed ([P,128,4] words) and, optionally, in the
 // reference's byte-per-element form; the pool is shared by all heads of a batch element.
 //
-// Three small kernels: (1) one CTA per (batch, Q block) classifies the row of tiles, compacts the
-// listed KV blocks in ascending order for head 0 and counts its PARTIAL tiles; (2) one CTA turns the
-// counts into pool offsets; (3) one CTA per (batch, Q block) writes the pool tiles and replicates
-// the lists over the heads. All of it is HBM-write bound (the index tensors).
+// limit(q) never decreases inside the sequence, so the limits of a block are those of its first and last
+// row, the listed KV blocks are 0 .. limit_max / 128, the first (limit_min + 1) / 128 of them FULL, and
+// everything there is to know about a Q block takes one pass over the spans. One kernel therefore does
+// it all: a CTA works out its own Q block and, for the position of its PARTIAL tiles in the pool, the
+// PARTIAL counts of all Q blocks before it (the counts of a thread's share of them, summed over the CTA),
+// writes its pool tiles and the lists of a slice of the heads. HBM-write bound for long sequences (the index
+// tensors: 101 MB for a 4 x 32-head batch of 32K tokens), one launch latency for short ones.
 #include <cstdint>
 
 #include "../../include/omni_attn_sm100.h"
@@ -40,196 +43,143 @@ struct MaskParams {
   uint32_t* partial_bits;             // [capacity, 128, 4]
   uint8_t* partial_bool;              // [capacity, 128, 128] or null
   int32_t* num_partial_out;           // device int
-  int32_t* counts;                    // scratch [B * nq]
-  int32_t* bases;                     // scratch [B * nq]
   int B, M, H, seqlen, nq, capacity;
+  int heads_per_cta;                  // heads whose lists one CTA writes (grid z = slices of the heads)
+  bool vec4;                          // list rows are 16-byte aligned
 };
 
-// limit of row q (-1 = the row attends nothing) and whether it is a plain causal row
-__device__ __forceinline__ int row_limit(const MaskParams& p, int b, int q, bool& plain) {
-  plain = true;
-  if (q >= p.seqlen) {
-    plain = false;
-    return -1;
-  }
+// limit of row q (-1 = the row attends nothing)
+__device__ __forceinline__ int row_limit(const MaskParams& p, int b, int q) {
+  if (q >= p.seqlen) return -1;
   int lim = q;
   const int32_t* m = p.modality_positions + static_cast<long long>(b) * p.M * 3;
   for (int i = 0; i < p.M; ++i) {
     const int off = __ldg(m + 3 * i + 1);
     const int len = __ldg(m + 3 * i + 2);
-    if (len > 0 && q >= off) {
-      lim = max(lim, off + len - 1);
-      if (q < off + len) plain = false;
-    }
+    if (len > 0 && q >= off) lim = max(lim, off + len - 1);
   }
   return min(lim, p.seqlen - 1);
 }
 
-__device__ __forceinline__ int tile_type(int lim_min, int lim_max, bool causal_block, int qb, int kb) {
-  const int k0 = kb * kBlock;
-  if (lim_max < k0) return kTypeMasked;
-  if (lim_min >= k0 + kBlock - 1) return kTypeFull;
-  if (kb == qb && causal_block) return kTypeCausal;
-  return kTypePartial;
+// One Q block: KV blocks [0, n_full) are FULL, [n_full, n_listed) PARTIAL, except that the diagonal one is
+// CAUSAL when every row of the block is a plain causal row (no row inside a span).
+struct BlockShape {
+  int n_full, n_listed;
+  bool causal_diag;
+  __device__ __forceinline__ bool diag_in_range(int qb) const { return causal_diag && qb >= n_full && qb < n_listed; }
+  __device__ __forceinline__ int partials(int qb) const { return max(0, n_listed - n_full) - (diag_in_range(qb) ? 1 : 0); }
+};
+
+__device__ __forceinline__ BlockShape block_shape(const MaskParams& p, int b, int qb) {
+  const int q0 = qb * kBlock, q1 = q0 + kBlock - 1;
+  const int last = min(q1, p.seqlen - 1);   // last row of the block that exists
+  int lim0 = q0, lim1 = last;
+  bool causal = q1 < p.seqlen;
+  const int32_t* m = p.modality_positions + static_cast<long long>(b) * p.M * 3;
+  for (int i = 0; i < p.M; ++i) {
+    const int off = __ldg(m + 3 * i + 1);
+    const int len = __ldg(m + 3 * i + 2);
+    if (len <= 0) continue;
+    if (q0 >= off) lim0 = max(lim0, off + len - 1);
+    if (last >= off) lim1 = max(lim1, off + len - 1);
+    if (max(off, q0) <= min(off + len - 1, q1)) causal = false;
+  }
+  const int lim_min = q1 < p.seqlen ? min(lim0, p.seqlen - 1) : -1;         // rows past the end attend nothing
+  const int lim_max = q0 < p.seqlen ? min(lim1, p.seqlen - 1) : -1;
+  BlockShape s;
+  s.n_full = (lim_min + 1) / kBlock;
+  s.n_listed = lim_max < 0 ? 0 : lim_max / kBlock + 1;
+  s.causal_diag = causal;
+  return s;
 }
 
-// block-wide min / max / and over 128 threads
-__device__ __forceinline__ void block_limits(int lim, bool plain_and_causal, int* smem, int& lim_min, int& lim_max,
-                                             bool& causal_block) {
-  int mn = lim, mx = lim;
-  int ok = plain_and_causal ? 1 : 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = min(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
-    mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    ok &= __shfl_xor_sync(0xFFFFFFFFu, ok, o);
-  }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    smem[w] = mn;
-    smem[4 + w] = mx;
-    smem[8 + w] = ok;
-  }
-  __syncthreads();
-  lim_min = min(min(smem[0], smem[1]), min(smem[2], smem[3]));
-  lim_max = max(max(smem[4], smem[5]), max(smem[6], smem[7]));
-  causal_block = (smem[8] & smem[9] & smem[10] & smem[11]) != 0;
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(kMaskThreads) mask_classify_kernel(const MaskParams p) {
-  __shared__ int red[12];
-  __shared__ int warp_tot[4], warp_part[4];
+__global__ void __launch_bounds__(kMaskThreads) mask_build_kernel(const MaskParams p) {
+  __shared__ int part[kMaskThreads / 32];
   const int qb = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
-  bool plain;
-  const int q = qb * kBlock + t;
-  const int lim = row_limit(p, b, q, plain);
-  int lim_min, lim_max;
-  bool causal_block;
-  block_limits(lim, plain && lim == q, red, lim_min, lim_max, causal_block);
+  const BlockShape own = block_shape(p, b, qb);
 
-  const long long row = (static_cast<long long>(b) * p.H * p.nq + qb) * p.nq;  // head 0
-  int n_listed = 0, n_partial = 0;
-  for (int base = 0; base < p.nq; base += kMaskThreads) {
-    const int kb = base + t;
-    const int type = kb < p.nq ? tile_type(lim_min, lim_max, causal_block, qb, kb) : kTypeMasked;
-    const bool listed = type != kTypeMasked, part = type == kTypePartial;
-    const uint32_t bl = __ballot_sync(0xFFFFFFFFu, listed), bp = __ballot_sync(0xFFFFFFFFu, part);
-    const int w = t >> 5, lane = t & 31;
-    if (lane == 0) {
-      warp_tot[w] = __popc(bl);
-      warp_part[w] = __popc(bp);
-    }
-    __syncthreads();
-    int pos = n_listed, ppos = n_partial;
-    for (int i = 0; i < w; ++i) {
-      pos += warp_tot[i];
-      ppos += warp_part[i];
-    }
-    pos += __popc(bl & ((1u << lane) - 1u));
-    ppos += __popc(bp & ((1u << lane) - 1u));
-    if (listed) {
-      p.kv_indices[row + pos] = kb;
-      p.block_mask_types[row + pos] = type;
-      p.partial_idx[row + pos] = part ? ppos : -1;   // position among this row's PARTIAL tiles for now
-    }
-    n_listed += warp_tot[0] + warp_tot[1] + warp_tot[2] + warp_tot[3];
-    n_partial += warp_part[0] + warp_part[1] + warp_part[2] + warp_part[3];
-    __syncthreads();
-  }
-  for (int i = n_listed + t; i < p.nq; i += kMaskThreads) {   // unused tail of the list
-    p.kv_indices[row + i] = 0;
-    p.block_mask_types[row + i] = kTypeMasked;
-    p.partial_idx[row + i] = -1;
-  }
-  if (t == 0) {
-    p.kv_num_blocks[(static_cast<long long>(b) * p.H) * p.nq + qb] = n_listed;
-    p.counts[b * p.nq + qb] = n_partial;
-  }
-}
-
-// exclusive scan of counts[B * nq] by one CTA (a few thousand entries at most)
-__global__ void __launch_bounds__(1024) mask_scan_kernel(const MaskParams p) {
-  __shared__ int part[1024];
-  const int n = p.B * p.nq;
-  const int per = (n + 1023) / 1024;
-  const int lo = min(n, static_cast<int>(threadIdx.x) * per), hi = min(n, lo + per);
-  int s = 0;
-  for (int i = lo; i < hi; ++i) s += p.counts[i];
-  part[threadIdx.x] = s;
+  // pool position of this block's first PARTIAL tile
+  int before = 0;
+  const int me = b * p.nq + qb;
+  for (int i = t; i < me; i += kMaskThreads) before += block_shape(p, i / p.nq, i % p.nq).partials(i % p.nq);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
+  if ((t & 31) == 0) part[t >> 5] = before;
   __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int run = part[threadIdx.x] - s;
-  for (int i = lo; i < hi; ++i) {
-    p.bases[i] = run;
-    run += p.counts[i];
-  }
-  if (threadIdx.x == 1023) *p.num_partial_out = part[1023];
-}
+  const int base = part[0] + part[1] + part[2] + part[3];
+  const bool diag = own.diag_in_range(qb);
 
-__global__ void __launch_bounds__(kMaskThreads) mask_emit_kernel(const MaskParams p) {
-  const int qb = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
-  bool plain;
-  const int lim = row_limit(p, b, qb * kBlock + t, plain);
-
-  const long long row = (static_cast<long long>(b) * p.H * p.nq + qb) * p.nq;  // head 0
-  const int n_listed = p.kv_num_blocks[(static_cast<long long>(b) * p.H) * p.nq + qb];
-  const int base = p.bases[b * p.nq + qb];
-  // pool tiles: thread t owns row t of every PARTIAL tile of this Q block
-  for (int i = 0; i < n_listed; ++i) {
-    const int local = p.partial_idx[row + i];
-    if (local < 0) continue;
-    const int pool = base + local;
-    if (pool >= p.capacity) continue;   // reported through num_partial_out > capacity
-    const int kb = p.kv_indices[row + i];
-    const int cnt = min(max(lim + 1 - kb * kBlock, 0), kBlock);   // allowed columns of this row
-    uint32_t w[4];
+  if (blockIdx.z == 0) {   // the pool, shared by the heads: thread t writes row t of every PARTIAL tile
+    const int lim = row_limit(p, b, qb * kBlock + t);
+    int pool = base;
+    for (int kb = own.n_full; kb < own.n_listed; ++kb) {
+      if (diag && kb == qb) continue;
+      const int slot = pool++;
+      if (slot >= p.capacity) break;   // reported through num_partial_out > capacity
+      const int cnt = min(max(lim + 1 - kb * kBlock, 0), kBlock);   // allowed columns of this row
+      uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int d = cnt - 32 * j;
-      w[j] = d >= 32 ? 0xFFFFFFFFu : (d <= 0 ? 0u : ((1u << d) - 1u));
-    }
-    reinterpret_cast<uint4*>(p.partial_bits)[static_cast<size_t>(pool) * kBlock + t] = make_uint4(w[0], w[1], w[2], w[3]);
-    if (p.partial_bool != nullptr) {
-      uint4* dst = reinterpret_cast<uint4*>(p.partial_bool + (static_cast<size_t>(pool) * kBlock + t) * kBlock);
+      for (int j = 0; j < 4; ++j) {
+        const int d = cnt - 32 * j;
+        w[j] = d >= 32 ? 0xFFFFFFFFu : (d <= 0 ? 0u : ((1u << d) - 1u));
+      }
+      reinterpret_cast<uint4*>(p.partial_bits)[static_cast<size_t>(slot) * kBlock + t] = make_uint4(w[0], w[1], w[2], w[3]);
+      if (p.partial_bool != nullptr) {
+        uint4* dst = reinterpret_cast<uint4*>(p.partial_bool + (static_cast<size_t>(slot) * kBlock + t) * kBlock);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        uint32_t x[4];
+        for (int j = 0; j < 8; ++j) {
+          uint32_t x[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int c0 = 16 * j + 4 * k;
-          x[k] = (c0 < cnt ? 1u : 0u) | (c0 + 1 < cnt ? 0x100u : 0u) | (c0 + 2 < cnt ? 0x10000u : 0u) |
-                 (c0 + 3 < cnt ? 0x1000000u : 0u);
+          for (int k = 0; k < 4; ++k) {
+            const int c0 = 16 * j + 4 * k;
+            x[k] = (c0 < cnt ? 1u : 0u) | (c0 + 1 < cnt ? 0x100u : 0u) | (c0 + 2 < cnt ? 0x10000u : 0u) |
+                   (c0 + 3 < cnt ? 0x1000000u : 0u);
+          }
+          dst[j] = make_uint4(x[0], x[1], x[2], x[3]);
         }
-        dst[j] = make_uint4(x[0], x[1], x[2], x[3]);
+      }
+    }
+    if (t == 0 && me == p.B * p.nq - 1) *p.num_partial_out = base + own.partials(qb);
+  }
+
+  // the lists, for this CTA's heads
+  const int h0 = blockIdx.z * p.heads_per_cta, h1 = min(p.H, h0 + p.heads_per_cta);
+  auto entry = [&](int i, int& idx, int& typ, int& pi) {
+    const bool listed = i < own.n_listed;
+    const bool part_tile = listed && i >= own.n_full && !(diag && i == qb);
+    idx = listed ? i : 0;
+    typ = !listed ? kTypeMasked : (i < own.n_full ? kTypeFull : (part_tile ? kTypePartial : kTypeCausal));
+    pi = part_tile ? base + (i - own.n_full) - (diag && i > qb ? 1 : 0) : -1;
+  };
+  const long long head_stride = static_cast<long long>(p.nq) * p.nq;
+  const long long row0 = (static_cast<long long>(b) * p.H * p.nq + qb) * p.nq;
+  if (p.vec4) {
+    for (int i = 4 * t; i < p.nq; i += 4 * kMaskThreads) {
+      int4 idx, typ, pi;
+      entry(i, idx.x, typ.x, pi.x);
+      entry(i + 1, idx.y, typ.y, pi.y);
+      entry(i + 2, idx.z, typ.z, pi.z);
+      entry(i + 3, idx.w, typ.w, pi.w);
+      for (int h = h0; h < h1; ++h) {
+        const long long at = row0 + h * head_stride + i;
+        *reinterpret_cast<int4*>(p.kv_indices + at) = idx;
+        *reinterpret_cast<int4*>(p.block_mask_types + at) = typ;
+        *reinterpret_cast<int4*>(p.partial_idx + at) = pi;
+      }
+    }
+  } else {
+    for (int i = t; i < p.nq; i += kMaskThreads) {
+      int idx, typ, pi;
+      entry(i, idx, typ, pi);
+      for (int h = h0; h < h1; ++h) {
+        const long long at = row0 + h * head_stride + i;
+        p.kv_indices[at] = idx;
+        p.block_mask_types[at] = typ;
+        p.partial_idx[at] = pi;
       }
     }
   }
-  __syncthreads();
-  // final pool indices for head 0, then the same list for every other head
-  for (int i = t; i < p.nq; i += kMaskThreads) {
-    const int kvb = p.kv_indices[row + i];
-    const int typ = p.block_mask_types[row + i];
-    int pi = p.partial_idx[row + i];
-    if (pi >= 0) pi += base;
-    p.partial_idx[row + i] = pi;
-    for (int h = 1; h < p.H; ++h) {
-      const long long r2 = row + static_cast<long long>(h) * p.nq * p.nq;
-      p.kv_indices[r2 + i] = kvb;
-      p.block_mask_types[r2 + i] = typ;
-      p.partial_idx[r2 + i] = pi;
-    }
-  }
-  if (t == 0) {
-    for (int h = 1; h < p.H; ++h) {
-      p.kv_num_blocks[(static_cast<long long>(b) * p.H + h) * p.nq + qb] = n_listed;
-    }
-  }
+  for (int h = h0 + t; h < h1; h += kMaskThreads) p.kv_num_blocks[(static_cast<long long>(b) * p.H + h) * p.nq + qb] = own.n_listed;
 }
 
 }  // namespace
@@ -265,13 +215,18 @@ extern "C" int omni_attn_build_mask_sm100(const int32_t* modality_positions, int
   p.partial_bits = partial_bits;
   p.partial_bool = partial_bool_or_null;
   p.num_partial_out = num_partial_out;
-  p.counts = static_cast<int32_t*>(scratch);
-  p.bases = p.counts + static_cast<long long>(B) * nq;
   p.B = B; p.M = M; p.H = H; p.seqlen = seqlen; p.nq = nq; p.capacity = partial_capacity;
+  const uintptr_t lists = reinterpret_cast<uintptr_t>(kv_indices) | reinterpret_cast<uintptr_t>(block_mask_types) |
+                          reinterpret_cast<uintptr_t>(partial_idx);
+  p.vec4 = nq % 4 == 0 && (lists & 15u) == 0;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-  const dim3 grid(nq, B);
-  mask_classify_kernel<<<grid, kMaskThreads, 0, st>>>(p);
-  mask_scan_kernel<<<1, 1024, 0, st>>>(p);
-  mask_emit_kernel<<<grid, kMaskThreads, 0, st>>>(p);
+  // Slices of the heads: enough CTAs to keep the memory system busy with a few (batch, Q block) pairs, but no
+  // more than that, since every slice repeats the counting of the blocks before its own.
+  const long long blocks = static_cast<long long>(nq) * B;
+  int slices = static_cast<int>(blocks >= 592 ? 1 : 592 / blocks);
+  if (slices > H) slices = H;
+  p.heads_per_cta = (H + slices - 1) / slices;
+  const dim3 grid(nq, B, (H + p.heads_per_cta - 1) / p.heads_per_cta);
+  mask_build_kernel<<<grid, kMaskThreads, 0, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? OMNI_OK : OMNI_ERR_CUDA;
 }
