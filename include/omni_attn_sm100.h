@@ -139,6 +139,21 @@ int omni_attn_fwd_ex_sm100(const void* q, const void* k, const void* v, void* o,
                            int32_t* device_status_or_null, float softcap, void* scratch_or_null,
                            long long scratch_bytes);
 
+/* omni_attn_fwd_ex_sm100 for tensors that are not padded in memory.
+ *  rows      rows a (batch, head) has in q, k, v, o and lse: seqlen_orig <= rows <= seqlen_padded. The rows
+ *            between rows and seqlen_padded are never touched: tiles that reach beyond the end are filled with
+ *            zeros by the copy unit and nothing is written there. rows == seqlen_padded is
+ *            omni_attn_fwd_ex_sm100. The reference pads the three inputs on the host instead
+ *            (omni-attn-mma/omni_attn_torch.py:1261-1284). */
+int omni_attn_fwd_rows_sm100(const void* q, const void* k, const void* v, void* o, float* lse_or_null,
+                             const int32_t* kv_num_blocks, const int32_t* kv_indices,
+                             const int32_t* block_mask_types, const int32_t* partial_idx_or_null,
+                             const uint8_t* partial_bool_or_null, const uint32_t* partial_bits_or_null, int B,
+                             int H, int seqlen_padded, int seqlen_orig, int head_dim, int q_block, int kv_block,
+                             int max_blocks, int num_partial, int dtype, float scale, void* cuda_stream,
+                             int32_t* device_status_or_null, int rows, float softcap, void* scratch_or_null,
+                             long long scratch_bytes);
+
 /* Forward pass for callers that have no device memory to hand over and may not allocate any.
  * This entry point has no counterpart in the reference.
  *
@@ -287,6 +302,18 @@ int omni_attn_bwd_ex_sm100(const void* q, const void* k, const void* v, const vo
                            int head_dim, int q_block, int kv_block, int max_blocks, int num_partial, int dtype,
                            float scale, void* cuda_stream, int32_t* device_status_or_null, void* workspace,
                            long long workspace_bytes, float softcap);
+
+/* omni_attn_bwd_ex_sm100 for tensors that are not padded in memory: q, k, v, o, d_o, dq, dk, dv
+ * [B, H, rows, head_dim] and lse [B, H, rows] with seqlen_orig <= rows <= seqlen_padded, as in
+ * omni_attn_fwd_rows_sm100. The workspace is that of seqlen_padded. */
+int omni_attn_bwd_rows_sm100(const void* q, const void* k, const void* v, const void* o, const float* lse,
+                             const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_num_blocks,
+                             const int32_t* kv_indices, const int32_t* block_mask_types,
+                             const int32_t* partial_idx_or_null, const uint8_t* partial_bool_or_null,
+                             const uint32_t* partial_bits_or_null, int B, int H, int seqlen_padded, int seqlen_orig,
+                             int head_dim, int q_block, int kv_block, int max_blocks, int num_partial, int dtype,
+                             float scale, void* cuda_stream, int32_t* device_status_or_null, void* workspace,
+                             long long workspace_bytes, float softcap, int rows);
 
 /* Text for an OMNI_ERR_* code; the pointer is static storage. */
 const char* omni_attn_error_string(int code);

@@ -34,35 +34,16 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// [rows, head_dim] 16-bit row-major view of one of Q/K/V; box = 128 rows x 64 columns (128 bytes),
-// 128-byte swizzle, which is the layout the UMMA shared-memory descriptors of the kernels expect.
-int make_tile_map(CUtensorMap* tm, const void* base, long long rows, int head_dim, bool bf16) {
+// [BH, rows, head_dim] view of one of Q, K, V, dO; box = 128 rows x 64 columns (128 bytes) of one (batch,
+// head), 128-byte swizzle, the layout the UMMA shared-memory descriptors of the kernels expect. Rows beyond
+// the end of a head and columns beyond head_dim (head_dim 32) read as zeros.
+int make_tile_map(CUtensorMap* tm, const void* base, long long BH, int rows, int head_dim, bool bf16) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return OMNI_ERR_NO_DRIVER_ENTRY;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(head_dim) * 2};
-  const cuuint32_t box[2] = {64, 128};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    g_last_cuda_error = static_cast<int>(r);
-    return OMNI_ERR_CUDA;
-  }
-  return OMNI_OK;
-}
-
-// [BH, N, head_dim] view of one of Q/K/V for the forward kernels; box = 128 rows x 64 columns of one
-// (batch, head), 128-byte swizzle. Rows beyond N and columns beyond head_dim (head_dim 32) read as zeros.
-int make_tile_map_3d(CUtensorMap* tm, const void* base, long long BH, int seqlen, int head_dim, bool bf16) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return OMNI_ERR_NO_DRIVER_ENTRY;
-  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(seqlen),
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(rows),
                               static_cast<cuuint64_t>(BH)};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(head_dim) * 2,
-                                 static_cast<cuuint64_t>(head_dim) * 2 * static_cast<cuuint64_t>(seqlen)};
+                                 static_cast<cuuint64_t>(head_dim) * 2 * static_cast<cuuint64_t>(rows)};
   const cuuint32_t box[3] = {64, 128, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
@@ -152,11 +133,13 @@ int forward(bool simple, const void* q, const void* k, const void* v, void* o, f
             const int32_t* partial_idx, const uint8_t* partial_bool, const uint32_t* partial_bits, int B,
             int H, int seqlen_padded, int seqlen_orig, int head_dim, int q_block, int kv_block,
             int max_blocks, int num_partial, int dtype, float scale, void* stream, int32_t* status,
-            void* scratch, float softcap = 0.f) {
+            void* scratch, float softcap = 0.f, int rows = 0) {
   int rc = validate_forward(simple, q, k, v, o, kv_num_blocks, kv_indices, types, partial_bool, partial_bits, B, H,
                             seqlen_padded, seqlen_orig, head_dim, q_block, kv_block, max_blocks, num_partial, dtype,
                             scratch, softcap);
   if (rc != OMNI_OK) return rc;
+  if (rows == 0) rows = seqlen_padded;
+  if (rows < seqlen_orig || rows > seqlen_padded) return OMNI_ERR_SEQLEN;
   const long long BH = static_cast<long long>(B) * H;
   const bool bf16 = dtype == OMNI_DTYPE_BF16;
   // head_dim 32 is computed by the 64-wide kernels: the TMA unit reads the missing columns as zeros
@@ -164,11 +147,11 @@ int forward(bool simple, const void* q, const void* k, const void* v, void* o, f
   CUtensorMap tmQ, tmK, tmV;
   rc = bind_context();
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map_3d(&tmQ, q, BH, seqlen_padded, head_dim, bf16);
+  rc = make_tile_map(&tmQ, q, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map_3d(&tmK, k, BH, seqlen_padded, head_dim, bf16);
+  rc = make_tile_map(&tmK, k, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map_3d(&tmV, v, BH, seqlen_padded, head_dim, bf16);
+  rc = make_tile_map(&tmV, v, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
 
   FwdParams p;
@@ -185,7 +168,7 @@ int forward(bool simple, const void* q, const void* k, const void* v, void* o, f
   p.num_units = 0;
   p.o_aligned32 = (reinterpret_cast<uintptr_t>(o) & 31u) == 0 ? 1 : 0;
   p.BH = static_cast<int>(BH);
-  p.N = seqlen_padded;
+  p.N = rows;
   p.seqlen_orig = seqlen_orig;
   p.nq = (seqlen_padded + kBlock - 1) / kBlock;
   p.max_blocks = max_blocks;
@@ -222,7 +205,7 @@ int backward(const void* q, const void* k, const void* v, const void* o, const f
              const int32_t* types, const int32_t* partial_idx, const uint8_t* partial_bool,
              const uint32_t* partial_bits, int B, int H, int seqlen_padded, int seqlen_orig, int head_dim,
              int q_block, int kv_block, int max_blocks, int num_partial, int dtype, float scale, void* stream,
-             int32_t* status, void* workspace, long long workspace_bytes, float softcap = 0.f) {
+             int32_t* status, void* workspace, long long workspace_bytes, float softcap = 0.f, int rows = 0) {
   if (softcap < 0.f || softcap != softcap) return OMNI_ERR_SOFTCAP;
   if (q == nullptr || k == nullptr || v == nullptr || o == nullptr || lse == nullptr || d_o == nullptr ||
       dq == nullptr || dk == nullptr || dv == nullptr || kv_num_blocks == nullptr || kv_indices == nullptr ||
@@ -237,8 +220,9 @@ int backward(const void* q, const void* k, const void* v, const void* o, const f
   }
   if (B <= 0 || H <= 0 || max_blocks <= 0) return OMNI_ERR_SHAPE;
   const long long BH = static_cast<long long>(B) * H;
-  const long long rows = BH * seqlen_padded;
-  if (rows >= (1LL << 31) || BH > 65535) return OMNI_ERR_SHAPE;
+  if (rows == 0) rows = seqlen_padded;
+  if (rows < seqlen_orig || rows > seqlen_padded) return OMNI_ERR_SEQLEN;
+  if (BH * seqlen_padded >= (1LL << 31) || BH > 65535) return OMNI_ERR_SHAPE;
   if (num_partial < 0) return OMNI_ERR_PARTIAL;
   if (num_partial > 0 && partial_bool == nullptr && partial_bits == nullptr) return OMNI_ERR_PARTIAL;
   const int nq = seqlen_padded / kBlock;
@@ -254,13 +238,13 @@ int backward(const void* q, const void* k, const void* v, const void* o, const f
   CUtensorMap tmQ, tmK, tmV, tmdO;
   int rc = bind_context();
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map(&tmQ, q, rows, head_dim, bf16);
+  rc = make_tile_map(&tmQ, q, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map(&tmK, k, rows, head_dim, bf16);
+  rc = make_tile_map(&tmK, k, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map(&tmV, v, rows, head_dim, bf16);
+  rc = make_tile_map(&tmV, v, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
-  rc = make_tile_map(&tmdO, d_o, rows, head_dim, bf16);
+  rc = make_tile_map(&tmdO, d_o, BH, rows, head_dim, bf16);
   if (rc != OMNI_OK) return rc;
 
   BwdParams p;
@@ -275,7 +259,7 @@ int backward(const void* q, const void* k, const void* v, const void* o, const f
   p.f.status = status;
   p.f.unit_counter = nullptr;
   p.f.BH = static_cast<int>(BH);
-  p.f.N = seqlen_padded;
+  p.f.N = rows;
   p.f.seqlen_orig = seqlen_orig;
   p.f.nq = nq;
   p.f.max_blocks = max_blocks;
@@ -373,6 +357,23 @@ int omni_attn_fwd_ex_sm100(const void* q, const void* k, const void* v, void* o,
                        partial_idx_or_null, partial_bool_or_null, partial_bits_or_null, B, H,
                        seqlen_padded, seqlen_orig, head_dim, q_block, kv_block, max_blocks, num_partial,
                        dtype, scale, cuda_stream, device_status_or_null, scratch_or_null, softcap);
+}
+
+int omni_attn_fwd_rows_sm100(const void* q, const void* k, const void* v, void* o, float* lse_or_null,
+                             const int32_t* kv_num_blocks, const int32_t* kv_indices,
+                             const int32_t* block_mask_types, const int32_t* partial_idx_or_null,
+                             const uint8_t* partial_bool_or_null, const uint32_t* partial_bits_or_null, int B,
+                             int H, int seqlen_padded, int seqlen_orig, int head_dim, int q_block, int kv_block,
+                             int max_blocks, int num_partial, int dtype, float scale, void* cuda_stream,
+                             int32_t* device_status_or_null, int rows, float softcap, void* scratch_or_null,
+                             long long scratch_bytes) {
+  if (rows <= 0) return OMNI_ERR_SEQLEN;
+  if (softcap < 0.f || softcap != softcap) return OMNI_ERR_SOFTCAP;
+  if (scratch_or_null != nullptr && scratch_bytes < OMNI_ATTN_SCRATCH_BYTES) return OMNI_ERR_SCRATCH;
+  return omni::forward(false, q, k, v, o, lse_or_null, kv_num_blocks, kv_indices, block_mask_types,
+                       partial_idx_or_null, partial_bool_or_null, partial_bits_or_null, B, H,
+                       seqlen_padded, seqlen_orig, head_dim, q_block, kv_block, max_blocks, num_partial,
+                       dtype, scale, cuda_stream, device_status_or_null, scratch_or_null, softcap, rows);
 }
 
 int omni_attn_fwd_simple_sm100(const void* q, const void* k, const void* v, void* o,
@@ -544,6 +545,21 @@ int omni_attn_bwd_ex_sm100(const void* q, const void* k, const void* v, const vo
                         partial_idx_or_null, partial_bool_or_null, partial_bits_or_null, B, H, seqlen_padded,
                         seqlen_orig, head_dim, q_block, kv_block, max_blocks, num_partial, dtype, scale,
                         cuda_stream, device_status_or_null, workspace, workspace_bytes, softcap);
+}
+
+int omni_attn_bwd_rows_sm100(const void* q, const void* k, const void* v, const void* o, const float* lse,
+                             const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_num_blocks,
+                             const int32_t* kv_indices, const int32_t* block_mask_types,
+                             const int32_t* partial_idx_or_null, const uint8_t* partial_bool_or_null,
+                             const uint32_t* partial_bits_or_null, int B, int H, int seqlen_padded, int seqlen_orig,
+                             int head_dim, int q_block, int kv_block, int max_blocks, int num_partial, int dtype,
+                             float scale, void* cuda_stream, int32_t* device_status_or_null, void* workspace,
+                             long long workspace_bytes, float softcap, int rows) {
+  if (rows <= 0) return OMNI_ERR_SEQLEN;
+  return omni::backward(q, k, v, o, lse, d_o, dq, dk, dv, kv_num_blocks, kv_indices, block_mask_types,
+                        partial_idx_or_null, partial_bool_or_null, partial_bits_or_null, B, H, seqlen_padded,
+                        seqlen_orig, head_dim, q_block, kv_block, max_blocks, num_partial, dtype, scale,
+                        cuda_stream, device_status_or_null, workspace, workspace_bytes, softcap, rows);
 }
 
 const char* omni_attn_error_string(int code) {

@@ -9,6 +9,7 @@
 // bf16 is accepted as well as fp16, the launch goes to torch's current stream instead of the legacy default stream, and
 // `omni_attn_fwd` adds optional scale / log-sum-exp / status arguments; `omni_attn_bwd` is the backward pass.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -299,6 +300,215 @@ long long omni_attn_bwd_workspace(int B, int H, int seqlen_padded) {
   return omni_attn_bwd_workspace_bytes(B, H, seqlen_padded);
 }
 
+// -------------------------------------------------------------------------------------------------
+// The operator's own path. For short sequences a call is host time, so everything the Python operator
+// does per call happens here: argument checks, allocation of the results, the C-ABI call and, for
+// training, the autograd node. (Through Python and ctypes the host side of a forward took about 28 us and
+// of a forward + backward about 80 us; the kernels of a 512-token call take 15.)
+// -------------------------------------------------------------------------------------------------
+
+// Device-side form of one OmniBlockMask: int32 lists, bit-packed (or byte) pool. Built once per mask object
+// and device by the Python side, which keeps it on the mask. The copies were enqueued on the stream that
+// was current at construction; a call on another stream waits for them.
+struct DeviceMask : torch::CustomClassHolder {
+  torch::Tensor nb, idx, types, pidx, pbool, pbits;
+  int block = 0, num_partial = 0, padded = 0, B = 0, H = 0, nq = 0, max_blocks = 0;
+  c10::DeviceIndex device = -1;
+  cudaStream_t built_on = nullptr;
+  at::cuda::CUDAEvent ready;
+
+  DeviceMask(torch::Tensor nb_, torch::Tensor idx_, torch::Tensor types_, std::optional<torch::Tensor> pidx_,
+             std::optional<torch::Tensor> pbool_, std::optional<torch::Tensor> pbits_, int num_partial_, int block_,
+             int padded_)
+      : nb(std::move(nb_)), idx(std::move(idx_)), types(std::move(types_)), block(block_), num_partial(num_partial_),
+        padded(padded_) {
+    check_index(nb, "kv_num_blocks");
+    check_index(idx, "kv_indices");
+    check_index(types, "block_mask_types");
+    if (nb.dim() != 3 || idx.dim() != 4 || idx.size(0) != nb.size(0) || idx.size(1) != nb.size(1) ||
+        idx.size(2) != nb.size(2) || types.sizes() != idx.sizes()) {
+      fail("kv_num_blocks must be [B, H, nq]; kv_indices and block_mask_types [B, H, nq, max_blocks]");
+    }
+    if (pidx_.has_value()) {
+      pidx = *pidx_;
+      check_index(pidx, "partial_block_mask_indices");
+      if (pidx.sizes() != idx.sizes()) fail("partial_block_mask_indices must have the shape of kv_indices");
+    }
+    if (pbool_.has_value()) pbool = *pbool_;
+    if (pbits_.has_value()) pbits = *pbits_;
+    B = static_cast<int>(nb.size(0));
+    H = static_cast<int>(nb.size(1));
+    nq = static_cast<int>(nb.size(2));
+    max_blocks = static_cast<int>(idx.size(3));
+    device = static_cast<c10::DeviceIndex>(nb.get_device());
+    c10::cuda::CUDAGuard guard(device);
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    ready.record(stream);
+    built_on = stream.stream();
+  }
+
+  void order_after_build(const at::cuda::CUDAStream& stream) {
+    if (stream.stream() != built_on) ready.block(stream);
+  }
+  const int32_t* partial_idx_ptr() const { return pidx.defined() ? pidx.data_ptr<int32_t>() : nullptr; }
+  const uint8_t* partial_bool_ptr() const {
+    return pbool.defined() && pbool.numel() > 0 ? reinterpret_cast<const uint8_t*>(pbool.data_ptr<bool>()) : nullptr;
+  }
+  const uint32_t* partial_bits_ptr() const {
+    return pbits.defined() && pbits.numel() > 0 ? reinterpret_cast<const uint32_t*>(pbits.data_ptr<int32_t>()) : nullptr;
+  }
+};
+using MaskPtr = c10::intrusive_ptr<DeviceMask>;
+
+// Whether the native path takes the call as it is; what it does not take goes back to the Python side,
+// which states what is wrong with it.
+bool accepts(const DeviceMask& m, const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v) {
+  if (!q.is_cuda() || q.dim() != 4 || q.get_device() != m.device) return false;
+  const auto dtype = q.scalar_type();
+  if (dtype != torch::kHalf && dtype != torch::kBFloat16) return false;
+  if (k.scalar_type() != dtype || v.scalar_type() != dtype || k.device() != q.device() || v.device() != q.device()) return false;
+  if (k.sizes() != q.sizes() || v.sizes() != q.sizes()) return false;
+  const int64_t n = q.size(2), d = q.size(3);
+  if (q.size(0) != m.B || q.size(1) != m.H || (d != 32 && d != 64 && d != 128)) return false;
+  if (n <= 0 || (n + m.block - 1) / m.block * m.block != m.padded || m.padded / m.block != m.nq) return false;
+  return true;
+}
+
+int forward_call(DeviceMask& m, const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v,
+                 torch::Tensor& out, float* lse, double scale, double softcap) {
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  m.order_after_build(stream);
+  const int n = static_cast<int>(q.size(2));
+  return omni_attn_fwd_rows_sm100(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse,
+                                  m.nb.data_ptr<int32_t>(), m.idx.data_ptr<int32_t>(), m.types.data_ptr<int32_t>(),
+                                  m.partial_idx_ptr(), m.partial_bool_ptr(), m.partial_bits_ptr(), m.B, m.H, m.padded, n,
+                                  static_cast<int>(q.size(3)), m.block, m.block, m.max_blocks, m.num_partial,
+                                  q.scalar_type() == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16,
+                                  static_cast<float>(scale), stream.stream(), nullptr, n, static_cast<float>(softcap),
+                                  stream_scratch(q, stream.stream()), OMNI_ATTN_SCRATCH_BYTES);
+}
+
+// None: not a call for this path; an int: the C ABI's error code; else the output, or (output, lse).
+pybind11::object operator_forward(const MaskPtr& m, torch::Tensor q, torch::Tensor k, torch::Tensor v, double scale,
+                                  double softcap, bool want_lse) {
+  if (!accepts(*m, q, k, v)) return pybind11::none();
+  torch::Tensor out, lse;
+  int rc;
+  {
+    pybind11::gil_scoped_release nogil;
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(m->device);
+    q = q.contiguous();
+    k = k.contiguous();
+    v = v.contiguous();
+    out = at::empty(q.sizes(), q.options());
+    if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(torch::kFloat32));
+    rc = forward_call(*m, q, k, v, out, want_lse ? lse.data_ptr<float>() : nullptr, scale, softcap);
+  }
+  if (rc != OMNI_OK) return pybind11::int_(rc);
+  if (want_lse) return pybind11::make_tuple(out, lse);
+  return pybind11::cast(out);
+}
+
+void throw_rc(const char* what, int rc) {
+  std::ostringstream os;
+  os << what << ": " << omni_attn_error_string(rc) << " (code " << rc;
+  if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << omni_attn_last_cuda_error();
+  os << ")";
+  fail(os.str());
+}
+
+struct OmniAttentionFn : torch::autograd::Function<OmniAttentionFn> {
+  static torch::Tensor forward(torch::autograd::AutogradContext* ctx, const torch::Tensor& q, const torch::Tensor& k,
+                               const torch::Tensor& v, const MaskPtr& mask, double scale, double softcap) {
+    auto out = at::empty(q.sizes(), q.options());
+    auto lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(torch::kFloat32));
+    const int rc = forward_call(*mask, q, k, v, out, lse.data_ptr<float>(), scale, softcap);
+    if (rc != OMNI_OK) throw_rc("omni_attn", rc);
+    ctx->save_for_backward({q, k, v, out, lse});
+    ctx->saved_data["mask"] = c10::IValue::make_capsule(mask);
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["softcap"] = softcap;
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const torch::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4];
+    auto mask = c10::static_intrusive_pointer_cast<DeviceMask>(ctx->saved_data["mask"].toCapsule());
+    c10::cuda::CUDAGuard guard(mask->device);
+    const auto d_out = grads[0].contiguous();
+    auto dq = at::empty(q.sizes(), q.options()), dk = at::empty(q.sizes(), q.options()),
+         dv = at::empty(q.sizes(), q.options());
+    const long long need = omni_attn_bwd_workspace_bytes(mask->B, mask->H, mask->padded);
+    auto workspace = at::empty({need}, q.options().dtype(torch::kUInt8));
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    mask->order_after_build(stream);
+    const int n = static_cast<int>(q.size(2));
+    const int rc = omni_attn_bwd_rows_sm100(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), d_out.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), mask->nb.data_ptr<int32_t>(), mask->idx.data_ptr<int32_t>(),
+        mask->types.data_ptr<int32_t>(), mask->partial_idx_ptr(), mask->partial_bool_ptr(), mask->partial_bits_ptr(),
+        mask->B, mask->H, mask->padded, n, static_cast<int>(q.size(3)), mask->block, mask->block, mask->max_blocks,
+        mask->num_partial, q.scalar_type() == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16,
+        static_cast<float>(ctx->saved_data["scale"].toDouble()), stream.stream(), nullptr, workspace.data_ptr(), need,
+        static_cast<float>(ctx->saved_data["softcap"].toDouble()), n);
+    if (rc != OMNI_OK) throw_rc("omni_attn", rc);
+    return {dq, dk, dv, torch::Tensor(), torch::Tensor(), torch::Tensor()};
+  }
+};
+
+// None: not a call for this path; else the differentiable output. `m` has 128-blocks.
+pybind11::object operator_autograd(const MaskPtr& m, torch::Tensor q, torch::Tensor k, torch::Tensor v, double scale,
+                                   double softcap) {
+  if (m->block != 128 || !accepts(*m, q, k, v)) return pybind11::none();
+  torch::Tensor out;
+  {
+    pybind11::gil_scoped_release nogil;
+    c10::cuda::CUDAGuard guard(m->device);
+    out = OmniAttentionFn::apply(q.contiguous(), k.contiguous(), v.contiguous(), m, scale, softcap);
+  }
+  return pybind11::cast(out);
+}
+
+// Mask construction on the GPU (omni_attn_build_mask_sm100) with everything it needs allocated here and nothing
+// waited for. Inside a batch element the row limits never decrease, so its Q blocks have at most 2 * nq - 1
+// PARTIAL tiles between them, plus at most nq in a last block that the sequence ends in: that sizes the pool
+// without counting anything (6 KB per Q block).
+// Returns (mask, kv_num_blocks, kv_indices, block_mask_types, partial indices, bit pool, count).
+pybind11::object build_mask(torch::Tensor modality_positions, int B, int H, int seqlen, int padded, int device) {
+  torch::Tensor nb, idx, types, pidx, bits, count, scratch;
+  MaskPtr mask;
+  int rc;
+  {
+    pybind11::gil_scoped_release nogil;
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    const auto opt = torch::TensorOptions().dtype(torch::kInt32).device(torch::kCUDA, static_cast<c10::DeviceIndex>(device));
+    const auto mp = modality_positions.to(opt).contiguous();
+    const int64_t nq = padded / 128;
+    const int capacity = static_cast<int>(3 * nq * B);
+    nb = at::empty({B, H, nq}, opt);
+    idx = at::empty({B, H, nq, nq}, opt);
+    types = at::empty({B, H, nq, nq}, opt);
+    pidx = at::empty({B, H, nq, nq}, opt);
+    bits = at::empty({capacity, 128, 4}, opt);
+    count = at::empty({1}, opt);
+    scratch = at::empty({2 * B * nq}, opt);
+    rc = omni_attn_build_mask_sm100(mp.numel() > 0 ? mp.data_ptr<int32_t>() : nullptr, B, static_cast<int>(mp.size(1)), H,
+                                    seqlen, padded, nb.data_ptr<int32_t>(), idx.data_ptr<int32_t>(),
+                                    types.data_ptr<int32_t>(), pidx.data_ptr<int32_t>(),
+                                    reinterpret_cast<uint32_t*>(bits.data_ptr<int32_t>()), nullptr, capacity,
+                                    count.data_ptr<int32_t>(), scratch.data_ptr<int32_t>(),
+                                    static_cast<long long>(scratch.numel()) * 4, at::cuda::getCurrentCUDAStream().stream());
+    if (rc == OMNI_OK) {
+      mask = c10::make_intrusive<DeviceMask>(nb, idx, types, pidx, std::nullopt, bits, capacity, 128, padded);
+    }
+  }
+  if (rc != OMNI_OK) return pybind11::int_(rc);
+  return pybind11::make_tuple(mask, nb, idx, types, pidx, bits, count);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -327,6 +537,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("has_partial"), pybind11::arg("workspace"), pybind11::arg("scale") = pybind11::none(),
         pybind11::arg("status") = pybind11::none(), pybind11::arg("partial_bits") = pybind11::none(),
         pybind11::arg("softcap") = 0.0);
+  pybind11::class_<DeviceMask, MaskPtr>(m, "DeviceMask", "device-side form of a block mask")
+      .def(pybind11::init([](torch::Tensor nb, torch::Tensor idx, torch::Tensor types, std::optional<torch::Tensor> pidx,
+                             std::optional<torch::Tensor> pbool, std::optional<torch::Tensor> pbits, int num_partial,
+                             int block, int padded) {
+        return c10::make_intrusive<DeviceMask>(nb, idx, types, pidx, pbool, pbits, num_partial, block, padded);
+      }));
+  m.def("operator_forward", &operator_forward, "the operator's forward on a DeviceMask");
+  m.def("operator_autograd", &operator_autograd, "the operator's differentiable forward on a DeviceMask");
+  m.def("build_mask", &build_mask, "block mask of an interleaved sequence, built on the GPU");
   m.def("omni_attn_bwd_workspace_bytes", &omni_attn_bwd_workspace, "bytes of workspace omni_attn_bwd needs",
         pybind11::arg("B"), pybind11::arg("H"), pybind11::arg("seqlen_padded"));
 }

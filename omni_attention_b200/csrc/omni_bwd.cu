@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(128) omni_bwd_prep_kernel(const BwdParams p) {
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int kWords = D / 64;   // 32-bit words (2 elements) per lane
   for (int rr = 0; rr < 32; ++rr) {
+    if (qb * kBlock + warp * 32 + rr >= p.f.N) break;   // the last tile of an unpadded tensor
     const long long row = static_cast<long long>(bh) * p.f.N + qb * kBlock + warp * 32 + rr;
     // rows are d_real elements long (head_dim 32 runs on the 64-wide instantiation: the upper lanes idle)
     const long long pitch = static_cast<long long>(p.f.d_real) * 2;
@@ -116,9 +117,9 @@ __global__ void __launch_bounds__(128) omni_bwd_prep_kernel(const BwdParams p) {
 // Pieces shared by the two tile kernels.
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ void bwd_load_tile(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int y) {
+__device__ __forceinline__ void bwd_load_tile(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int y, int bh) {
 #pragma unroll
-  for (int c = 0; c < BwdCfg<D>::kChunks; ++c) tma_load_2d(dst + c * BwdCfg<D>::kChunkBytes, tm, bar, c * 64, y);
+  for (int c = 0; c < BwdCfg<D>::kChunks; ++c) tma_load_3d(dst + c * BwdCfg<D>::kChunkBytes, tm, bar, c * 64, y, bh);
 }
 
 // The issuing thread runs ahead of the tensor pipe by about eight MMAs as long as it spends less time on
@@ -168,10 +169,10 @@ __device__ __forceinline__ void bwd_mma_ts_split(uint32_t d_tmem, uint32_t a_reg
 }
 
 // One accumulator row (32-column chunks [kFirstChunk, kEndChunk) of it) out of TMEM, times `mul`, as
-// 16-bit values to global memory (zeros when `have_acc` is false).
+// 16-bit values to global memory (zeros when `have_acc` is false; nothing when the row is not in memory).
 template <int D, bool BF16, int kFirstChunk = 0, int kEndChunk = D / 32>
 __device__ __forceinline__ void bwd_store_row(uint32_t taddr_row, bool have_acc, float mul, void* base,
-                                              long long row_index, int d_real) {
+                                              long long row_index, int d_real, bool in_memory) {
   // rows of the output are d_real elements long; accumulator columns beyond that (head_dim 32 on the
   // 64-wide instantiation) are zero and are not stored
   uint4* dst = reinterpret_cast<uint4*>(static_cast<char*>(base) + row_index * (static_cast<long long>(d_real) * 2));
@@ -192,7 +193,9 @@ __device__ __forceinline__ void bwd_store_row(uint32_t taddr_row, bool have_acc,
       w[j] = pack2<BF16>(__uint_as_float(r[2 * j]) * mul, __uint_as_float(r[2 * j + 1]) * mul);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dst[4 * c + j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+    for (int j = 0; j < 4; ++j) {
+      if (in_memory) dst[4 * c + j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+    }
   }
 }
 
@@ -374,21 +377,21 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // =========================== TMA producer ====================================================
     if (n_vis > 0) {
       mbar_expect_tx(bar_kv, 2 * Cfg::kTileBytes);
-      const int y = static_cast<int>(row0 + kvb * kBlock);
-      bwd_load_tile<D>(sK, &tmK, bar_kv, y);
-      bwd_load_tile<D>(sV, &tmV, bar_kv, y);
+      const int y = kvb * kBlock;
+      bwd_load_tile<D>(sK, &tmK, bar_kv, y, bh);
+      bwd_load_tile<D>(sV, &tmV, bar_kv, y, bh);
     }
     for (int i = 0; i < n_vis; ++i) {
       const int stage = i & 1;
-      const int y = static_cast<int>(row0 + static_cast<int>(vis_s[i]) * kBlock);
+      const int y = static_cast<int>(vis_s[i]) * kBlock;
       const uint32_t prev = static_cast<uint32_t>(((i >> 1) - 1) & 1);   // parity of the stage's previous use
       // Q first: it is needed first (S^T opens the visit) although its stage is freed last (by dK)
       if (i >= 2) mbar_wait(bar_dkdone + 8 * stage, prev, abort_flag, p.f.status, 55);
       mbar_expect_tx(bar_q + 8 * stage, Cfg::kTileBytes);
-      bwd_load_tile<D>(sQ + stage * Cfg::kTileBytes, &tmQ, bar_q + 8 * stage, y);
+      bwd_load_tile<D>(sQ + stage * Cfg::kTileBytes, &tmQ, bar_q + 8 * stage, y, bh);
       if (i >= 2) mbar_wait(bar_dvdone + 8 * stage, prev, abort_flag, p.f.status, 56);
       mbar_expect_tx(bar_do + 8 * stage, Cfg::kTileBytes);
-      bwd_load_tile<D>(sdO + stage * Cfg::kTileBytes, &tmdO, bar_do + 8 * stage, y);
+      bwd_load_tile<D>(sdO + stage * Cfg::kTileBytes, &tmdO, bar_do + 8 * stage, y, bh);
     }
   } else if (warp == kBwdIssuerWarp && elect_one()) {
     // =========================== MMA issuer ======================================================
@@ -581,9 +584,9 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     const long long out_row = row0 + k_abs;
     if (half == 0) {
-      bwd_store_row<D, BF16>(tdV + lane_base, n_vis > 0, 1.f, p.dv, out_row, p.f.d_real);
+      bwd_store_row<D, BF16>(tdV + lane_base, n_vis > 0, 1.f, p.dv, out_row, p.f.d_real, k_abs < p.f.N);
     } else {
-      bwd_store_row<D, BF16>(tdK + lane_base, n_vis > 0, p.f.scale, p.dk, out_row, p.f.d_real);
+      bwd_store_row<D, BF16>(tdK + lane_base, n_vis > 0, p.f.scale, p.dk, out_row, p.f.d_real, k_abs < p.f.N);
     }
   }
 
@@ -710,19 +713,19 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // =========================== TMA producer ====================================================
     if (n_vis > 0) {
       mbar_expect_tx(bar_qdo, 2 * Cfg::kTileBytes);
-      const int y = static_cast<int>(row0 + qb * kBlock);
-      bwd_load_tile<D>(sQ, &tmQ, bar_qdo, y);
-      bwd_load_tile<D>(sdO, &tmdO, bar_qdo, y);
+      const int y = qb * kBlock;
+      bwd_load_tile<D>(sQ, &tmQ, bar_qdo, y, bh);
+      bwd_load_tile<D>(sdO, &tmdO, bar_qdo, y, bh);
     }
     for (int j = 0; j < n_vis; ++j) {
-      const int y = static_cast<int>(row0 + static_cast<int>(vis_s[j]) * kBlock);
+      const int y = static_cast<int>(vis_s[j]) * kBlock;
       const int ks = j % 3, vs = j & 1;
       if (j >= 3) mbar_wait(bar_kfree + 8 * ks, static_cast<uint32_t>((j / 3 - 1) & 1), abort_flag, p.f.status, 65);
       mbar_expect_tx(bar_k + 8 * ks, Cfg::kTileBytes);
-      bwd_load_tile<D>(sK + ks * Cfg::kTileBytes, &tmK, bar_k + 8 * ks, y);
+      bwd_load_tile<D>(sK + ks * Cfg::kTileBytes, &tmK, bar_k + 8 * ks, y, bh);
       if (j >= 2) mbar_wait(bar_vfree + 8 * vs, static_cast<uint32_t>(((j >> 1) - 1) & 1), abort_flag, p.f.status, 66);
       mbar_expect_tx(bar_v + 8 * vs, Cfg::kTileBytes);
-      bwd_load_tile<D>(sV + vs * Cfg::kTileBytes, &tmV, bar_v + 8 * vs, y);
+      bwd_load_tile<D>(sV + vs * Cfg::kTileBytes, &tmV, bar_v + 8 * vs, y, bh);
     }
   } else if (warp == kBwdIssuerWarp && elect_one()) {
     // =========================== MMA issuer ======================================================
@@ -844,9 +847,9 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_after();
     }
     if (half == 0) {
-      bwd_store_row<D, BF16, 0, D / 64>(tdQ + lane_base, n_vis > 0, p.f.scale, p.dq, my_row, p.f.d_real);
+      bwd_store_row<D, BF16, 0, D / 64>(tdQ + lane_base, n_vis > 0, p.f.scale, p.dq, my_row, p.f.d_real, q_abs < p.f.N);
     } else {
-      bwd_store_row<D, BF16, D / 64, D / 32>(tdQ + lane_base, n_vis > 0, p.f.scale, p.dq, my_row, p.f.d_real);
+      bwd_store_row<D, BF16, D / 64, D / 32>(tdQ + lane_base, n_vis > 0, p.f.scale, p.dq, my_row, p.f.d_real, q_abs < p.f.N);
     }
   }
 

@@ -42,9 +42,9 @@ struct FwdParams {
   int32_t* status;                // device status word or null
   int32_t* unit_counter;          // zeroed int32 in caller scratch for dynamic unit hand-out, or null
   int BH;
-  int N;            // padded sequence length (multiple of 128; of 64 with blk64)
+  int N;            // rows a (batch, head) has in memory: the padded sequence length, or fewer (>= seqlen_orig)
   int seqlen_orig;  // unpadded length
-  int nq;           // ceil(N / 128): 128-row tiles per (batch, head)
+  int nq;           // 128-row tiles per (batch, head): ceil(padded length / 128)
   int max_blocks;
   int num_partial;
   float scale;           // softmax scale
@@ -57,8 +57,8 @@ struct FwdParams {
   int o_aligned32;       // output base address is 32-byte aligned (256-bit stores allowed)
   int d_real;            // head_dim of the tensors in memory: 32, 64 or 128 (32 is computed as 64 with the
                          // missing columns read as zeros by the TMA unit); row pitch of o is d_real * 2 bytes
-  int blk64;             // 1: the lists, types and partial pool are in 64x64 blocks (N a multiple of 64)
-  int nq_lists;          // Q blocks in the lists: N / 64 with blk64, else nq
+  int blk64;             // 1: the lists, types and partial pool are in 64x64 blocks
+  int nq_lists;          // Q blocks in the lists: padded length / 64 with blk64, else nq
   long long wait_cycles; // cycle budget of one bounded wait in the forward kernels
 };
 

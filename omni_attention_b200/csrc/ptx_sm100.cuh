@@ -146,19 +146,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tm) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
 }
-// x = element coordinate along the innermost (head_dim) axis; x * 2 bytes must be a multiple of 16.
-__device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* tm, uint32_t bar,
-                                            int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, "
-      "%4}], [%2];"
-      ::"r"(smem_dst),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-
-// The same for a [BH, N, D] view: x along head_dim, y = row inside the (batch, head), z = batch*head.
-// Rows at y >= N and columns at x >= D of the tensor are filled with zeros.
+// [BH, N, D] view: x = element coordinate along head_dim (x * 2 bytes must be a multiple of 16), y = row
+// inside the (batch, head), z = batch * head. Rows at y >= N and columns at x >= D of the tensor are filled
+// with zeros.
 __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* tm, uint32_t bar,
                                             int x, int y, int z) {
   asm volatile(

@@ -8,9 +8,11 @@ Same contract as the reference's wrappers ``omni_attention_shared_kv`` and sibli
   * the launch goes to torch's current stream and nothing synchronises the device (the reference
     calls ``torch.cuda.synchronize()`` after every launch, :666);
   * ``return_lse=True`` also returns the log-sum-exp rows;
-  * mask tensors are converted / bit-packed once per mask object and cached on it.
-The call goes through the C ABI of ``libomni_attn_sm100.so`` with raw device pointers. There is no
-CPU or PyTorch fallback: a missing library or a non-CUDA tensor raises.
+  * mask tensors are converted / bit-packed once per mask object and cached on it;
+  * tensors are not padded: the kernels take [B, H, N, D] of any N as it lies in memory.
+``omni_attention`` and ``omni_attention_autograd`` go through the in-tree ``omni_attn`` extension module (one
+native call per operator call), everything else through the C ABI of ``libomni_attn_sm100.so`` with raw
+device pointers. There is no CPU or PyTorch fallback: a missing library or a non-CUDA tensor raises.
 """
 from __future__ import annotations
 
@@ -22,7 +24,7 @@ from typing import Optional, Tuple, Union
 import torch
 from torch import Tensor
 
-from .block_mask import OmniBlockMask
+from .block_mask import OmniBlockMask, retile_block_mask
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libomni_attn_sm100.so")
 _lib = None
@@ -32,6 +34,7 @@ ABI_SYMBOLS = (
     "omni_attn_fwd_sm100",
     "omni_attn_fwd_scratch_sm100",
     "omni_attn_fwd_ex_sm100",
+    "omni_attn_fwd_rows_sm100",
     "omni_attn_fwd_noalloc_sm100",
     "omni_attn_fwd_simple_sm100",
     "omni_attn_pack_partial_masks_sm100",
@@ -42,6 +45,7 @@ ABI_SYMBOLS = (
     "omni_attn_bwd_workspace_bytes",
     "omni_attn_bwd_sm100",
     "omni_attn_bwd_ex_sm100",
+    "omni_attn_bwd_rows_sm100",
     "omni_attn_error_string",
     "omni_attn_last_cuda_error",
     "omni_attn_abi_version",
@@ -140,50 +144,30 @@ def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, s
     table (O(B*N*M) integer arithmetic). The kernels write the pool bit-packed, which is what the
     attention kernels read; the container's byte-per-element ``partial_block_masks`` is expanded from it
     only if somebody reads that field."""
-    from .block_mask import _limits_from_modality_tensor, count_partial_tiles
-
-    lib = load_library()
-    limits, plain = _limits_from_modality_tensor(modality_positions, int(seq_len), int(padded))
-    need = count_partial_tiles(limits, plain)
-    mp = modality_positions.to(device=device, dtype=torch.int32).contiguous()
-    M = int(mp.shape[1])
-    nq = padded // 128
-    nb = torch.empty(batch, nheads, nq, dtype=torch.int32, device=device)
-    idx = torch.empty(batch, nheads, nq, nq, dtype=torch.int32, device=device)
-    typ = torch.empty_like(idx)
-    pidx = torch.empty_like(idx)
-    count = torch.zeros(1, dtype=torch.int32, device=device)
-    scratch = torch.empty(2 * batch * nq, dtype=torch.int32, device=device)
-    bits = torch.empty(max(need, 1), 128, 4, dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
-        stream = torch.cuda.current_stream().cuda_stream
-        _check(lib.omni_attn_build_mask_sm100(_ptr(mp), batch, M, nheads, int(seq_len), int(padded), nb.data_ptr(),
-                                              idx.data_ptr(), typ.data_ptr(), pidx.data_ptr(), bits.data_ptr(), None,
-                                              need, count.data_ptr(), scratch.data_ptr(), scratch.numel() * 4,
-                                              stream))
-        ready = torch.cuda.Event()
-        ready.record(torch.cuda.current_stream(device))
-        built_on = torch.cuda.current_stream(device).cuda_stream
-    bits = bits[:need]
+    res = _native().build_mask(modality_positions, batch, nheads, int(seq_len), int(padded),
+                               device.index if device.index is not None else torch.cuda.current_device())
+    if isinstance(res, int):
+        _check(res)
+    mask, nb, idx, typ, pidx, bits, count = res
+    device = nb.device
+    built_on = torch.cuda.current_stream(device)
     bm = OmniBlockMask(nb, idx, typ, padded, padded, 128, 128, pidx, None)
 
     def expand_pool() -> Tensor:
-        # first read of the reference-shaped pool: also the place where the host count is checked
-        # against the one the kernels made (reading it waits for the GPU, which this read does anyway)
+        # first read of the reference-shaped pool: waits for the GPU to learn how many tiles there are
         cur = torch.cuda.current_stream(device)
-        if cur.cuda_stream != built_on:
-            cur.wait_event(ready)
-        if int(count.item()) != need:
-            raise RuntimeError(f"mask builder: the kernels counted {int(count.item())} PARTIAL tiles, the host {need}")
+        if cur != built_on:
+            cur.wait_stream(built_on)
+        need = int(count.item())
         shifts = torch.arange(32, dtype=torch.int32, device=device)
-        return ((bits.unsqueeze(-1) >> shifts) & 1).bool().view(need, 128, 128)
+        return ((bits[:need].unsqueeze(-1) >> shifts) & 1).bool().view(need, 128, 128)
 
     bm.set_lazy_partial_pool(expand_pool)
-    # what the attention calls use; a caller that asks for the byte-per-element pool (pack_bits=False)
-    # gets it through the container's field, expanded then
-    bm._cache[(str(device), True)] = {"nb": nb, "idx": idx, "typ": typ, "pidx": pidx, "pbool": None,
-                                      "pbits": bits if need > 0 else None, "num_partial": need,
-                                      "ready": ready, "stream": built_on}
+    bm._cache[device.index] = mask
+    # what omni_attention_forward_out uses; a caller that asks for the byte-per-element pool
+    # (pack_bits=False) gets it through the container's field, expanded then
+    bm._cache[(str(device), True)] = {"nb": nb, "idx": idx, "typ": typ, "pidx": pidx, "pbool": None, "pbits": bits,
+                                      "num_partial": int(bits.shape[0]), "ready": None, "built_on": built_on}
     return bm
 
 
@@ -195,8 +179,8 @@ def _device_mask(bm: OmniBlockMask, device: torch.device, pack_bits: bool) -> di
         # The copies and the pack kernel were enqueued on the stream that was current when the entry
         # was built; a call on another stream must not run ahead of them.
         cur = torch.cuda.current_stream(device)
-        if hit.get("ready") is not None and cur.cuda_stream != hit.get("stream"):
-            cur.wait_event(hit["ready"])
+        if cur != hit["built_on"]:
+            cur.wait_event(hit["ready"]) if hit["ready"] is not None else cur.wait_stream(hit["built_on"])
         return hit
     cv = lambda t: t.to(device=device, dtype=torch.int32).contiguous()
     d = {"nb": cv(bm.kv_num_blocks), "idx": cv(bm.kv_indices), "typ": cv(bm.block_mask_types),
@@ -213,9 +197,34 @@ def _device_mask(bm: OmniBlockMask, device: torch.device, pack_bits: bool) -> di
     with torch.cuda.device(device):
         d["ready"] = torch.cuda.Event()
         d["ready"].record(torch.cuda.current_stream(device))
-        d["stream"] = torch.cuda.current_stream(device).cuda_stream
+        d["built_on"] = torch.cuda.current_stream(device)
     bm._cache[key] = d
     return d
+
+
+_ext = None
+
+
+def _native():
+    """The in-tree extension module (built by ``omni_attention_b200.build``)."""
+    global _ext
+    if _ext is None:
+        from . import install_reference_module
+
+        _ext = install_reference_module()
+    return _ext
+
+
+def _native_mask(bm: OmniBlockMask, device: torch.device):
+    """The mask in the extension module's form, made once per mask object and device; None for a mask or a
+    device it does not take, which the caller's own checks then name."""
+    if device.type != "cuda" or bm.Q_BLOCK_SIZE not in (64, 128) or bm.KV_BLOCK_SIZE != bm.Q_BLOCK_SIZE or bm.kv_len != bm.q_len:
+        return None
+    d = _device_mask(bm, device, True)
+    mask = _native().DeviceMask(d["nb"], d["idx"], d["typ"], d["pidx"], d["pbool"], d["pbits"], d["num_partial"],
+                                bm.Q_BLOCK_SIZE, bm.q_len)
+    bm._cache[device.index] = mask
+    return mask
 
 
 def omni_attention_forward_out(q: Tensor, k: Tensor, v: Tensor, out: Tensor, block_mask: OmniBlockMask,
@@ -223,16 +232,7 @@ def omni_attention_forward_out(q: Tensor, k: Tensor, v: Tensor, out: Tensor, blo
                                status: Optional[Tensor] = None, kernel: str = "ws", pack_bits: bool = True,
                                softcap: Optional[float] = None) -> None:
     """Launch the forward on padded, contiguous CUDA tensors; writes ``out`` (and ``lse``) in place."""
-    if not (q.is_cuda and k.is_cuda and v.is_cuda and out.is_cuda):
-        raise OmniAttnError("omni_attention needs CUDA tensors (there is no CPU path)")
-    if q.dtype not in (torch.float16, torch.bfloat16):
-        raise OmniAttnError(f"unsupported dtype {q.dtype}: fp16 or bf16")
-    for t in (k, v, out):
-        if t.dtype != q.dtype or t.shape != q.shape:
-            raise OmniAttnError("q, k, v, out must share dtype and shape (Q_len == KV_len)")
-    for t in (q, k, v, out):
-        if not t.is_contiguous():
-            raise OmniAttnError("q, k, v, out must be contiguous")
+    _check_tensors(q, k, v, out)
     B, H, N, D = q.shape
     m = _device_mask(block_mask, q.device, pack_bits)
     nq = N // block_mask.Q_BLOCK_SIZE if block_mask.Q_BLOCK_SIZE else 0
@@ -282,49 +282,45 @@ def _scratch_for(device: torch.device, stream: int) -> Tensor:
     return t
 
 
-def _pad_to_block(x: Tensor, block: int) -> Tuple[Tensor, int]:
-    n = x.shape[2]
-    rem = (-n) % block
-    if rem == 0:
-        return x, n
-    return torch.nn.functional.pad(x, (0, 0, 0, rem)), n
+def _pad_to_block(x: Tensor, block: int) -> Tensor:
+    rem = (-x.shape[2]) % block
+    return (x if rem == 0 else torch.nn.functional.pad(x, (0, 0, 0, rem))).contiguous()
 
 
-def _prepare(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask, scale: Optional[float],
-             for_backward: bool = False):
-    """Shape checks and padding. The forward kernels take everything the reference's launchers accept
-    (omni-attn-mma/mma/omni_attn_shared_kv.cu:725-741: head_dim 32/64/128, blocks 64 or 128) as it is,
-    so all that happens here is the reference wrapper's zero-padding of the sequence to a multiple of
-    the mask's block size (omni_attn_torch.py:1261-1284).
-
-    The backward kernels take 128x128 blocks only; with ``for_backward`` a 64x64-block mask is
-    re-expressed on 128-tiles once (quadrant by quadrant, cached on the mask object).
-    Returns padded contiguous q, k, v, the mask to use, the scale, and the original length / head_dim."""
+def _check_shapes(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask) -> None:
+    """What the operator asks of its arguments, as errors (the reference launchers' checks,
+    omni-attn-mma/mma/omni_attn_shared_kv.cu:725-741: head_dim 32/64/128, blocks 64 or 128)."""
     B, H, Q, D = query.shape
     if key.shape != (B, H, Q, D) or value.shape != (B, H, Q, D):
         raise OmniAttnError(f"key/value shape must equal query shape {(B, H, Q, D)} (Q_len == KV_len)")
     if D not in (32, 64, 128):
         raise ValueError(f"Unsupported head_dim={D}. Supported: 32, 64, 128.")
-    sizes = (block_mask.Q_BLOCK_SIZE, block_mask.KV_BLOCK_SIZE)
-    if sizes not in ((64, 64), (128, 128)):
+    if (block_mask.Q_BLOCK_SIZE, block_mask.KV_BLOCK_SIZE) not in ((64, 64), (128, 128)):
         raise ValueError("Unsupported block size: Q_BLOCK_SIZE and KV_BLOCK_SIZE must both be 64 or both be 128.")
-    if for_backward:
-        if sizes == (64, 64):
-            hit = block_mask._cache.get("retiled128")
-            if hit is None:
-                from .block_mask import retile_block_mask
-
-                hit = retile_block_mask(block_mask, 128)
-                block_mask._cache["retiled128"] = hit
-            block_mask = hit
-    blk = block_mask.Q_BLOCK_SIZE
-    qp, n_orig = _pad_to_block(query, blk)
-    kp, _ = _pad_to_block(key, blk)
-    vp, _ = _pad_to_block(value, blk)
-    if qp.shape[2] != block_mask.q_len or kp.shape[2] != block_mask.kv_len:
+    padded = -(-Q // block_mask.Q_BLOCK_SIZE) * block_mask.Q_BLOCK_SIZE
+    if padded != block_mask.q_len or padded != block_mask.kv_len:
         raise OmniAttnError(
-            f"padded length {qp.shape[2]} does not match the mask's q_len/kv_len ({block_mask.q_len}/{block_mask.kv_len})")
-    return qp.contiguous(), kp.contiguous(), vp.contiguous(), block_mask, scale, n_orig, D
+            f"padded length {padded} does not match the mask's q_len/kv_len ({block_mask.q_len}/{block_mask.kv_len})")
+
+
+def _check_tensors(q: Tensor, k: Tensor, v: Tensor, out: Tensor, need_contiguous: bool = True) -> None:
+    if not (q.is_cuda and k.is_cuda and v.is_cuda and out.is_cuda):
+        raise OmniAttnError("omni_attention needs CUDA tensors (there is no CPU path)")
+    if q.dtype not in (torch.float16, torch.bfloat16):
+        raise OmniAttnError(f"unsupported dtype {q.dtype}: fp16 or bf16")
+    for t in (k, v, out):
+        if t.dtype != q.dtype or t.shape != q.shape or t.device != q.device:
+            raise OmniAttnError("q, k, v, out must share dtype, shape and device (Q_len == KV_len)")
+    for t in (q, k, v, out):
+        if need_contiguous and not t.is_contiguous():
+            raise OmniAttnError("q, k, v, out must be contiguous")
+
+
+def _refuse(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask) -> None:
+    """Names what is wrong with a call the extension module did not take."""
+    _check_shapes(query, key, value, block_mask)
+    _check_tensors(query, key, value, query, need_contiguous=False)
+    raise OmniAttnError(f"kv_num_blocks shape {tuple(block_mask.kv_num_blocks.shape)} does not fit q {tuple(query.shape)}")
 
 
 def omni_attention(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask,
@@ -338,8 +334,22 @@ def omni_attention(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBl
     tanh soft-cap to the scaled scores before masking (transfusion_pytorch/transfusion.py:358-364). ``check_status=True`` synchronises and
     raises if the kernel reported a bounded-wait timeout or an out-of-range block index.
     """
-    B, H = query.shape[:2]
-    qp, kp, vp, block_mask, scale, n_orig, d_orig = _prepare(query, key, value, block_mask, scale)
+    if kernel == "ws" and not check_status:
+        mask = block_mask._cache.get(query.get_device())
+        if mask is None:
+            mask = _native_mask(block_mask, query.device)
+        res = None
+        if mask is not None:
+            res = _native().operator_forward(mask, query, key, value, scale or 0.0, softcap or 0.0, return_lse)
+        if res is None:
+            _refuse(query, key, value, block_mask)
+        if isinstance(res, int):
+            _check(res)
+        return res
+    # the plain kernel, the fixed unit assignment, the status word: padded as the C ABI's basic entries want it
+    _check_shapes(query, key, value, block_mask)
+    B, H, n_orig = query.shape[:3]
+    qp, kp, vp = (_pad_to_block(t, block_mask.Q_BLOCK_SIZE) for t in (query, key, value))
     out = torch.empty_like(qp)
     lse = torch.empty(B, H, qp.shape[2], dtype=torch.float32, device=qp.device) if return_lse else None
     status = torch.zeros(1, dtype=torch.int32, device=qp.device) if check_status else None
@@ -350,7 +360,7 @@ def omni_attention(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBl
             raise OmniAttnError(f"kernel gave up waiting (status {code:#x}); output is not valid")
         if code & 0xFF == STATUS_BAD_INDEX:
             raise OmniAttnError("kv_indices holds a block id outside [0, num_kv_blocks); the entry was skipped")
-    out = out[:, :, :n_orig, :d_orig]
+    out = out[:, :, :n_orig]
     if return_lse:
         return out, lse[:, :, :n_orig]
     return out
@@ -395,38 +405,26 @@ def omni_attention_backward_out(q: Tensor, k: Tensor, v: Tensor, out: Tensor, ls
     _check(rc)
 
 
-class _OmniAttentionFn(torch.autograd.Function):
-    """Forward and backward kernels as one differentiable op on padded tensors."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, block_mask, seqlen_orig, scale, softcap):
-        out = torch.empty_like(q)
-        lse = torch.empty(q.shape[0], q.shape[1], q.shape[2], dtype=torch.float32, device=q.device)
-        omni_attention_forward_out(q, k, v, out, block_mask, seqlen_orig, scale, lse, softcap=softcap)
-        ctx.save_for_backward(q, k, v, out, lse)
-        ctx.block_mask, ctx.seqlen_orig, ctx.scale, ctx.softcap = block_mask, seqlen_orig, scale, softcap
-        return out
-
-    @staticmethod
-    def backward(ctx, d_out):
-        q, k, v, out, lse = ctx.saved_tensors
-        d_out = d_out.contiguous()
-        if ctx.seqlen_orig < q.shape[2]:
-            d_out = d_out.clone()
-            d_out[:, :, ctx.seqlen_orig:] = 0   # padded rows take no part but must be finite
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        omni_attention_backward_out(q, k, v, out, lse, d_out, dq, dk, dv, ctx.block_mask, ctx.seqlen_orig, ctx.scale,
-                                    softcap=ctx.softcap)
-        return dq, dk, dv, None, None, None, None
-
-
 def omni_attention_autograd(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask,
                             scale: Optional[float] = None, softcap: Optional[float] = None) -> Tensor:
     """``omni_attention`` for training: same inputs and output, differentiable with respect to
     query, key and value (the gradients come from omni_attn_bwd_sm100 / omni_attn_bwd_ex_sm100)."""
-    qp, kp, vp, block_mask, scale, n_orig, d_orig = _prepare(query, key, value, block_mask, scale, for_backward=True)
-    out = _OmniAttentionFn.apply(qp, kp, vp, block_mask, n_orig, scale, softcap if softcap else None)
-    return out[:, :, :n_orig, :d_orig]
+    if block_mask.Q_BLOCK_SIZE == 64 and block_mask.KV_BLOCK_SIZE == 64:
+        # the backward kernels take 128-blocks: re-expressed quadrant by quadrant, once per mask object
+        hit = block_mask._cache.get("retiled128")
+        if hit is None:
+            _check_shapes(query, key, value, block_mask)
+            hit = block_mask._cache["retiled128"] = retile_block_mask(block_mask, 128)
+        block_mask = hit
+    mask = block_mask._cache.get(query.get_device())
+    if mask is None:
+        mask = _native_mask(block_mask, query.device)
+    out = None
+    if mask is not None:
+        out = _native().operator_autograd(mask, query, key, value, scale or 0.0, softcap or 0.0)
+    if out is None:
+        _refuse(query, key, value, block_mask)
+    return out
 
 
 def default_scale(head_dim: int) -> float:

@@ -1,0 +1,73 @@
+"""The operator on tensors whose length is no multiple of the block size, as they lie in memory, and the
+one-kernel mask builder at the edges of its blocks."""
+import pytest
+import torch
+
+from omni_attention_b200 import (block_mask_from_row_limits, create_omni_block_mask_from_modality_positions as build_mask,
+                                 omni_attention, omni_attention_autograd, retile_block_mask)
+from omni_attention_b200.ops import omni_attention_backward_out, omni_attention_forward_out
+
+pytestmark = pytest.mark.gpu
+
+
+def _limits(n, padded, g):
+    """Row limits of a causal mask with one span attended in both directions."""
+    lim = torch.arange(padded).clamp(max=n - 1)
+    a = int(torch.randint(0, n, (1,), generator=g))
+    b = min(n, a + int(torch.randint(1, 200, (1,), generator=g)))
+    lim[a:b] = b - 1
+    lim[n:] = n - 1
+    return lim.view(1, padded)
+
+
+@pytest.mark.parametrize("block", [128, 64])
+@pytest.mark.parametrize("n", [1, 63, 65, 127, 129, 200, 383, 385])
+@pytest.mark.parametrize("D,dtype", [(32, torch.float16), (64, torch.bfloat16), (128, torch.bfloat16)])
+def test_unpadded_tensors_give_the_bits_of_padded_ones(cuda_device, n, D, dtype, block):
+    """Forward, log-sum-exp and gradients of [1, 3, n, D] tensors against the same call on zero-padded
+    copies through the padded entry points: the same tiles reach the tensor cores, so the bits are equal. Three
+    heads back to back, so that reading past a head's end would read the next head."""
+    g = torch.Generator().manual_seed(1000 * D + n)
+    padded = -(-n // block) * block
+    H = 3
+    bm = block_mask_from_row_limits(_limits(n, padded, g), H, block=block)
+    q, k, v, do = ((torch.randn(1, H, n, D, generator=g)).to(dtype).to(cuda_device) for _ in range(4))
+    pad = lambda t, to: torch.nn.functional.pad(t, (0, 0, 0, to - n)).contiguous()
+    out, lse = omni_attention(q, k, v, bm, return_lse=True)
+    assert out.shape == q.shape and out.is_contiguous() and lse.shape == q.shape[:3]
+    po, plse = torch.empty(1, H, padded, D, dtype=dtype, device=cuda_device), torch.empty(1, H, padded, device=cuda_device)
+    omni_attention_forward_out(pad(q, padded), pad(k, padded), pad(v, padded), po, bm, n, lse=plse)
+    assert torch.equal(out, po[:, :, :n]) and torch.equal(lse, plse[:, :, :n])
+
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    got = torch.autograd.grad(omni_attention_autograd(*leaves, bm), leaves, do)
+    bm128 = bm if block == 128 else retile_block_mask(bm, 128)
+    p128 = bm128.q_len
+    pq, pk, pv, pdo = (pad(t, p128) for t in (q, k, v, do))
+    po, plse = torch.empty_like(pq), torch.empty(1, H, p128, device=cuda_device)
+    omni_attention_forward_out(pq, pk, pv, po, bm128, n, lse=plse)
+    want = [torch.empty_like(pq) for _ in range(3)]
+    omni_attention_backward_out(pq, pk, pv, po, plse, pdo, *want, bm128, n)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b[:, :, :n])
+
+
+@pytest.mark.parametrize("n", [100, 128, 129, 512, 640, 1023, 1025, 2048])
+def test_mask_builder_at_block_edges(cuda_device, n):
+    """Spans that begin and end at, one before and one after block boundaries, overlap, are empty or reach past
+    the end, for lengths with and without a rest: lists, types and tiles of the CPU builder."""
+    spans = [[(0, 0, 1)], [(0, 127, 2)], [(0, 128, 128)], [(0, 129, 126)], [(0, 0, 128), (0, 128, 1)],
+             [(0, 60, 300), (0, 100, 50), (0, 255, 2)], [(0, 5, 0), (0, n - 1, 1)], [(0, max(0, n - 130), 500)], [(0, 3, 4 * n)]]
+    m = max(len(s) for s in spans)
+    mp = torch.tensor([s + [(0, 0, 0)] * (m - len(s)) for s in spans], dtype=torch.int32)
+    B, H = len(spans), 3
+    cpu = build_mask(mp, B, H, n, n)
+    gpu = build_mask(mp.to(cuda_device), B, H, n, n, device=cuda_device)
+    for name in ("kv_num_blocks", "kv_indices", "block_mask_types"):
+        assert torch.equal(getattr(gpu, name).cpu(), getattr(cpu, name)), name
+    sel = cpu.partial_block_mask_indices >= 0
+    gi = gpu.partial_block_mask_indices.cpu()
+    assert torch.equal(gi >= 0, sel)
+    assert gpu.partial_block_masks.shape == cpu.partial_block_masks.shape
+    assert torch.equal(gpu.partial_block_masks.cpu()[gi[sel].long()],
+                       cpu.partial_block_masks[cpu.partial_block_mask_indices[sel].long()])
