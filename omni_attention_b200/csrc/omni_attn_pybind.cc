@@ -388,6 +388,14 @@ int forward_call(DeviceMask& m, const torch::Tensor& q, const torch::Tensor& k, 
                                   stream_scratch(q, stream.stream()), OMNI_ATTN_SCRATCH_BYTES);
 }
 
+// Contiguous, and for a length that is no multiple of the block (callers of such lengths may pass any view)
+// 16-byte aligned: TMA reads rows where they lie. Other lengths keep the C ABI's refusal of unaligned tensors.
+torch::Tensor packed(const torch::Tensor& t, const DeviceMask& m) {
+  auto c = t.contiguous();
+  const bool ragged = c.size(2) != m.padded;
+  return ragged && reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 != 0 ? c.clone() : c;
+}
+
 // None: not a call for this path; an int: the C ABI's error code; else the output, or (output, lse).
 pybind11::object operator_forward(const MaskPtr& m, torch::Tensor q, torch::Tensor k, torch::Tensor v, double scale,
                                   double softcap, bool want_lse) {
@@ -398,9 +406,9 @@ pybind11::object operator_forward(const MaskPtr& m, torch::Tensor q, torch::Tens
     pybind11::gil_scoped_release nogil;
     at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::CUDAGuard guard(m->device);
-    q = q.contiguous();
-    k = k.contiguous();
-    v = v.contiguous();
+    q = packed(q, *m);
+    k = packed(k, *m);
+    v = packed(v, *m);
     out = at::empty(q.sizes(), q.options());
     if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(torch::kFloat32));
     rc = forward_call(*m, q, k, v, out, want_lse ? lse.data_ptr<float>() : nullptr, scale, softcap);
@@ -438,7 +446,7 @@ struct OmniAttentionFn : torch::autograd::Function<OmniAttentionFn> {
     const torch::Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4];
     auto mask = c10::static_intrusive_pointer_cast<DeviceMask>(ctx->saved_data["mask"].toCapsule());
     c10::cuda::CUDAGuard guard(mask->device);
-    const auto d_out = grads[0].contiguous();
+    const auto d_out = packed(grads[0], *mask);
     auto dq = at::empty(q.sizes(), q.options()), dk = at::empty(q.sizes(), q.options()),
          dv = at::empty(q.sizes(), q.options());
     const long long need = omni_attn_bwd_workspace_bytes(mask->B, mask->H, mask->padded);
@@ -467,7 +475,7 @@ pybind11::object operator_autograd(const MaskPtr& m, torch::Tensor q, torch::Ten
   {
     pybind11::gil_scoped_release nogil;
     c10::cuda::CUDAGuard guard(m->device);
-    out = OmniAttentionFn::apply(q.contiguous(), k.contiguous(), v.contiguous(), m, scale, softcap);
+    out = OmniAttentionFn::apply(packed(q, *m), packed(k, *m), packed(v, *m), m, scale, softcap);
   }
   return pybind11::cast(out);
 }

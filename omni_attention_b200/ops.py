@@ -316,6 +316,11 @@ def _check_tensors(q: Tensor, k: Tensor, v: Tensor, out: Tensor, need_contiguous
             raise OmniAttnError("q, k, v, out must be contiguous")
 
 
+def _cap(softcap: Optional[float]) -> float:
+    """The native calls' form of ``softcap``: 0 = none, which is also what a value that is not positive means."""
+    return float(softcap) if softcap is not None and softcap > 0 else 0.0
+
+
 def _refuse(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBlockMask) -> None:
     """Names what is wrong with a call the extension module did not take."""
     _check_shapes(query, key, value, block_mask)
@@ -340,7 +345,7 @@ def omni_attention(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBl
             mask = _native_mask(block_mask, query.device)
         res = None
         if mask is not None:
-            res = _native().operator_forward(mask, query, key, value, scale or 0.0, softcap or 0.0, return_lse)
+            res = _native().operator_forward(mask, query, key, value, scale or 0.0, _cap(softcap), return_lse)
         if res is None:
             _refuse(query, key, value, block_mask)
         if isinstance(res, int):
@@ -421,7 +426,7 @@ def omni_attention_autograd(query: Tensor, key: Tensor, value: Tensor, block_mas
         mask = _native_mask(block_mask, query.device)
     out = None
     if mask is not None:
-        out = _native().operator_autograd(mask, query, key, value, scale or 0.0, softcap or 0.0)
+        out = _native().operator_autograd(mask, query, key, value, scale or 0.0, _cap(softcap))
     if out is None:
         _refuse(query, key, value, block_mask)
     return out

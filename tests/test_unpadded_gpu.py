@@ -71,3 +71,33 @@ def test_mask_builder_at_block_edges(cuda_device, n):
     assert gpu.partial_block_masks.shape == cpu.partial_block_masks.shape
     assert torch.equal(gpu.partial_block_masks.cpu()[gi[sel].long()],
                        cpu.partial_block_masks[cpu.partial_block_mask_indices[sel].long()])
+
+
+@pytest.mark.parametrize("n", [200, 383])
+def test_views_that_start_at_any_element(cuda_device, n):
+    """A length that is no multiple of the block may come as a view at any element offset (the rows are copied
+    then, as padding copied them): outputs and gradients of the aligned copies."""
+    g = torch.Generator().manual_seed(n)
+    bm = block_mask_from_row_limits(_limits(n, -(-n // 128) * 128, g), 2)
+    shape = (1, 2, n, 64)
+    numel = 2 * n * 64
+    view = lambda off: torch.randn(numel + 8, generator=g).half().to(cuda_device)[off:off + numel].view(shape)
+    q, k, v, do = (view(off) for off in (1, 3, 4, 7))
+    assert torch.equal(omni_attention(q, k, v, bm), omni_attention(q.clone(), k.clone(), v.clone(), bm))
+
+    def grads(tensors, d_out):
+        leaves = [t.detach().requires_grad_(True) for t in tensors]
+        return torch.autograd.grad(omni_attention_autograd(*leaves, bm), leaves, d_out)
+
+    for a, b in zip(grads((q, k, v), do), grads([t.clone() for t in (q, k, v)], do.clone())):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("softcap", [0.0, -1.0, float("nan")])
+def test_a_cap_that_is_not_positive_is_none(cuda_device, softcap):
+    g = torch.Generator().manual_seed(5)
+    bm = block_mask_from_row_limits(_limits(256, 256, g), 1)
+    q, k, v = (torch.randn(1, 1, 256, 64, generator=g).half().to(cuda_device) for _ in range(3))
+    want = omni_attention(q, k, v, bm)
+    assert torch.equal(omni_attention(q, k, v, bm, softcap=softcap), want)
+    assert torch.equal(omni_attention_autograd(q, k, v, bm, softcap=softcap), want)
