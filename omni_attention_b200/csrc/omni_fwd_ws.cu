@@ -94,12 +94,17 @@ struct WsCfg {
   static constexpr int kPolyNum = (D == 128) ? 0 : 1;   // element pairs per group of kPolyDen on the FMA pipe
   static constexpr int kPolyDen = (D == 128) ? 1 : 4;
   // q_full[2] q_free ring_full[S] ring_empty[S] s_full[2] p_ready[2] p_half[2] done[2] o_free[2] tab_full[2]
-  // tab_empty[2] near_end drained
-  static constexpr int kNumBars = 3 + 2 * kStages + 15 + 1;
+  // tab_empty[2] near_end drained x_full[2] x_free[2]
+  static constexpr int kNumBars = 3 + 2 * kStages + 15 + 1 + 4;
   static constexpr int kBarBytes = (8 * kNumBars + 64 + 15) & ~15;   // barriers + a few control words; the table slots
                                                                      // behind them stay 16-byte aligned
   static constexpr int kFixedBytes = (2 + kStages) * kTileBytes + kBarBytes + 1024;   // + alignment slack
 };
+
+// Split form: what the two softmax groups of a tile hand each other at its end - 16 fp32 columns of the
+// 128 rows at a time, and each row's running maximum and sum - in shared memory behind the barriers.
+constexpr int kXchgCols = 16;
+constexpr int kXchgBytes = 2 * kXchgCols * kBlock * 4 + 2 * kBlock * 8;
 
 constexpr int kWsThreads = 384;
 // Register split made with setmaxnreg. The kernel is compiled for 168 registers per thread (the most
@@ -158,7 +163,7 @@ __device__ __forceinline__ void decode_unit(const FwdParams& p, int unit, int np
   bh = grp * G + rem % heads_here;
 }
 
-template <int D, bool BF16, bool SOFTCAP, bool B64>
+template <int D, bool BF16, bool SOFTCAP, bool B64, bool SPLIT>
 __global__ void __launch_bounds__(kWsThreads, 1)
 omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
@@ -187,10 +192,13 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t bar_tempty = bar_tfull + 16;                   // [2] unit table no longer needed (10 arrivals)
   const uint32_t bar_near = bar_tempty + 16;                    // the producer is within a few blocks of the unit's end
   const uint32_t bar_drain = bar_near + 8;                      // every MMA issued by this CTA has retired
+  const uint32_t bar_xfull = bar_drain + 8;                     // [2] split form: group's columns written (128 arrivals)
+  const uint32_t bar_xfree = bar_xfull + 16;                    // [2] ... and read by the other group (128 arrivals)
   int* misc = reinterpret_cast<int*>(bars + Cfg::kNumBars);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 0);
   volatile int* abort_flag = misc + 1;
-  uint8_t* slot_base = after_tiles + Cfg::kBarBytes;
+  float* xchg = reinterpret_cast<float*>(after_tiles + Cfg::kBarBytes);   // split form: [2][kXchgCols][128], (max, sum) [2][128]
+  uint8_t* slot_base = after_tiles + Cfg::kBarBytes + (SPLIT ? kXchgBytes : 0);
   const int slot_bytes = ws_slot_bytes(p.nq, B64);
   auto slot = [&](int k) -> UnitSlot {
     uint8_t* b = slot_base + (k & 1) * slot_bytes;
@@ -206,7 +214,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const int npairs = (p.nq + 1) >> 1;
+  const int npairs = SPLIT ? p.nq : (p.nq + 1) >> 1;   // units of a (batch, head): pairs of tiles, or tiles
   const long long wait_lim = p.wait_cycles;
 
   // ---- one-time set-up: barriers, tables, TMEM ---------------------------------------------------
@@ -226,6 +234,8 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(bar_ofree + 8 * g, 128);
       mbar_init(bar_tfull + 8 * g, 1);
       mbar_init(bar_tempty + 8 * g, 10);
+      mbar_init(bar_xfull + 8 * g, 128);
+      mbar_init(bar_xfree + 8 * g, 128);
     }
     mbar_init(bar_near, 1);
     mbar_init(bar_drain, 1);
@@ -271,12 +281,13 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t my_bar_p = bar_p + 8 * g;
     int n_tiles = 0;   // S tiles consumed so far over all units = phase count of the S and P barriers
     int n_units = 0;   // units in which this tile had work = phase count of its done barrier
+    int n_x = 0;       // split form: column chunks exchanged so far over all units = phase count of the exchange barriers
 
     for (int k = 0;; ++k) {
       const UnitSlot T = wait_table(k, 10 + g);
       const int n_sched = T.hdr->n_sched;
       if (n_sched < 0) break;
-      const uint32_t tab = smem_u32(T.tab[g]);
+      const uint32_t tab = smem_u32(T.tab[SPLIT ? 0 : g]);
       const uint32_t sched = smem_u32(T.sched);
       const int my_cnt = T.hdr->cnt[g];
       const int unit_bh = T.hdr->bh, unit_pair = T.hdr->pair;
@@ -353,7 +364,74 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         ++n_tiles;
       }
 
-      {
+      if constexpr (SPLIT) {
+        // ---- output of a tile whose KV blocks the two groups took in turn: each group finishes half of the
+        // columns, and gets the other group's share of them (and of the row's maximum and sum) through
+        // shared memory. O is handed back to the MMA issuer after the last chunk has been read. -------------
+        if (my_cnt > 0) {
+          mbar_wait_lim(bar_done + 8 * g, n_units & 1, abort_flag, p.status, 14 + g, wait_lim);
+          tc_fence_after();
+          ++n_units;
+        }
+        const int q_abs = unit_pair * kBlock + r;
+        const bool have_row = q_abs < p.N;
+        const long long row = static_cast<long long>(unit_bh) * p.N + q_abs;
+        float* x_mine = xchg + g * kXchgCols * kBlock + r;
+        const float* x_other = xchg + (g ^ 1) * kXchgCols * kBlock + r;
+        float2* ml = reinterpret_cast<float2*>(xchg + 2 * kXchgCols * kBlock);
+        float f_mine = 0.f, f_other = 0.f;   // what the two accumulators are multiplied by
+#pragma unroll
+        for (int c = 0; c < D / 2 / kXchgCols; ++c, ++n_x) {
+          const int col = g * (D / 2) + kXchgCols * c;   // finished here
+          uint32_t give[kXchgCols], own[kXchgCols];
+          if (my_cnt > 0) {   // uniform over the group
+            tmem_ld16(tO + (g ^ 1) * (D / 2) + kXchgCols * c, give);
+            tmem_ld16(tO + col, own);
+            tc_wait_ld();
+            if (c == D / 2 / kXchgCols - 1) {
+              tc_fence_before();
+              mbar_arrive(bar_ofree + 8 * g);   // the next unit may overwrite O now
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < kXchgCols; ++j) give[j] = own[j] = 0u;
+          }
+          if (n_x > 0) mbar_wait_lim(bar_xfree + 8 * g, (n_x - 1) & 1, abort_flag, p.status, 16 + g, wait_lim);
+          if (c == 0) ml[g * kBlock + r] = make_float2(st.M, st.l);
+#pragma unroll
+          for (int j = 0; j < kXchgCols; ++j) x_mine[j * kBlock] = __uint_as_float(give[j]);
+          mbar_arrive(bar_xfull + 8 * g);
+          mbar_wait_lim(bar_xfull + 8 * (g ^ 1), n_x & 1, abort_flag, p.status, 18 + g, wait_lim);
+          if (c == 0) {
+            const float2 o = ml[(g ^ 1) * kBlock + r];
+            const float M = fmaxf(st.M, o.x);
+            // both maxima are integers: the two factors are exact powers of two (0 for a group without keys)
+            const float a_mine = st.M == -INFINITY ? 0.f : ex2_approx(st.M - M);
+            const float a_other = o.x == -INFINITY ? 0.f : ex2_approx(o.x - M);
+            const float l = st.l * a_mine + o.y * a_other;
+            const bool empty = q_abs >= p.seqlen_orig || M == -INFINITY || !(l > 0.f);
+            const float inv = empty ? 0.f : 1.f / l;
+            f_mine = a_mine * inv;
+            f_other = a_other * inv;
+            if (g == 0 && have_row && p.lse != nullptr) {
+              p.lse[row] = empty ? -INFINITY : fmaf(M, 0.6931471805599453f, __logf(l));
+            }
+          }
+          uint32_t w[kXchgCols / 2];
+#pragma unroll
+          for (int j = 0; j < kXchgCols / 2; ++j) {
+            const float a = f_mine * __uint_as_float(own[2 * j]) + f_other * x_other[(2 * j) * kBlock];
+            const float b = f_mine * __uint_as_float(own[2 * j + 1]) + f_other * x_other[(2 * j + 1) * kBlock];
+            w[j] = pack2<BF16>(a, b);
+          }
+          mbar_arrive(bar_xfree + 8 * (g ^ 1));
+          if (have_row && col < p.d_real) {
+            char* d32 = static_cast<char*>(p.o) + row * (p.d_real * 2) + 2 * col;
+            reinterpret_cast<uint4*>(d32)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            reinterpret_cast<uint4*>(d32)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+          }
+        }
+      } else {
         // ---- output of the unit by the softmax group itself: O out of TMEM chunk by chunk, normalise,
         // store; O is handed back to the MMA issuer as soon as the last chunk has been read ----------
         if (my_cnt > 0) {
@@ -423,7 +501,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int n_sched = T.hdr->n_sched;
           if (n_sched < 0) break;
           const int bh = T.hdr->bh;
-          const int qbA = 2 * T.hdr->pair;
+          const int qbA = SPLIT ? T.hdr->pair : 2 * T.hdr->pair;
           if (*abort_flag) break;   // giving up: issue no further copies
           if (n_sched > 0) {
             // Q buffers are free once every S of the previous unit that used them is done.
@@ -436,7 +514,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
                 for (int c = 0; c < Cfg::kChunks; ++c) {
                   tma_load_3d(sQ0 + g * Cfg::kTileBytes + c * Cfg::kChunkBytes, &tmQ, bar_q + 8 * g, c * 64,
-                              (qbA + g) * kBlock, bh);
+                              (SPLIT ? qbA : qbA + g) * kBlock, bh);
                 }
               }
             }
@@ -578,7 +656,36 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           constexpr std::integral_constant<int, 0> tile_a{};
           constexpr std::integral_constant<int, 1> tile_b{};
 
-          if (n_sched > 0) {
+          if constexpr (SPLIT) {
+            // the two groups take the entries in turn; per group the order is the same: P*V(e), S(e + 2)
+            auto load_s = [&](uint32_t e) {
+              wait_full(2 * e);
+              tc_fence_after();
+              if (e & 1) {
+                issue_s(tile_b, e, no_peek);
+              } else {
+                issue_s(tile_a, e, no_peek);
+              }
+              release(2 * e);
+              if (static_cast<int>(e) + 1 == n_sched) tc_commit(bar_qfree);   // the last S of the unit has been issued
+            };
+            const uint32_t n = static_cast<uint32_t>(n_sched);
+            if (n > 0) {
+              issued_any = true;
+              load_s(0);
+              if (n > 1) load_s(1);
+            }
+            for (uint32_t e = 0; e < n && alive; ++e) {
+              wait_full(2 * e + 1);
+              if (e & 1) {
+                issue_pv(tile_b, e, false);
+              } else {
+                issue_pv(tile_a, e, false);
+              }
+              release(2 * e + 1);
+              if (e + 2 < n) load_s(e + 2);
+            }
+          } else if (n_sched > 0) {
             issued_any = true;
             uint32_t cur = lds_u16(sched);
             {  // prologue: scores of the first visited block
@@ -673,10 +780,10 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         int bh, pair;
         decode_unit(p, unit, npairs, bh, pair);
         const int tab_words = p.nq * ws_words_per_block(B64);
-        for (int i = lane; i < 2 * tab_words; i += 32) T.tab[0][i] = 0u;   // tile A's table, then tile B's
+        for (int i = lane; i < (SPLIT ? 1 : 2) * tab_words; i += 32) T.tab[0][i] = 0u;   // tile A's table, then tile B's
         __syncwarp();
-        build_tile_table<B64>(p, bh, 2 * pair, T.tab[0]);
-        build_tile_table<B64>(p, bh, 2 * pair + 1, T.tab[1]);
+        build_tile_table<B64>(p, bh, SPLIT ? pair : 2 * pair, T.tab[0]);
+        if constexpr (!SPLIT) build_tile_table<B64>(p, bh, 2 * pair + 1, T.tab[1]);
         __syncwarp();
         int n = 0, ca = 0, cb = 0;   // compact the visited KV blocks into an ascending list
         for (int base = 0; base < p.nq; base += 32) {
@@ -684,16 +791,22 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           bool a = false, b = false;
           if (kvb < p.nq) {
             a = tile_visits<B64>(smem_u32(T.tab[0]), kvb);
-            b = tile_visits<B64>(smem_u32(T.tab[1]), kvb);
+            if constexpr (!SPLIT) b = tile_visits<B64>(smem_u32(T.tab[1]), kvb);
           }
           const uint32_t any = __ballot_sync(0xFFFFFFFFu, a || b);
           ca += __popc(__ballot_sync(0xFFFFFFFFu, a));
           cb += __popc(__ballot_sync(0xFFFFFFFFu, b));
-          if (a || b) {
-            T.sched[n + __popc(any & ((1u << lane) - 1u))] =
-                static_cast<uint16_t>(kvb | (a ? kSchedA : 0) | (b ? kSchedB : 0));
+          const int at = n + __popc(any & ((1u << lane) - 1u));
+          if (SPLIT && a) {   // the groups take the blocks in turn
+            a = (at & 1) == 0;
+            b = !a;
           }
+          if (a || b) T.sched[at] = static_cast<uint16_t>(kvb | (a ? kSchedA : 0) | (b ? kSchedB : 0));
           n += __popc(any);
+        }
+        if constexpr (SPLIT) {
+          ca = (n + 1) >> 1;
+          cb = n >> 1;
         }
         if (lane == 0) {
           T.hdr->n_sched = n;
@@ -718,17 +831,35 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
 // Dynamic shared memory of one CTA for sequences of nq 128-row tiles.
 template <int D>
-static int ws_smem_bytes(int nq, bool b64) {
-  return WsCfg<D>::kFixedBytes + 2 * ws_slot_bytes(nq, b64);
+static int ws_smem_bytes(int nq, bool b64, bool split) {
+  return WsCfg<D>::kFixedBytes + 2 * ws_slot_bytes(nq, b64) + (split ? kXchgBytes : 0);
 }
 
 constexpr int kMaxSmemPerCta = 232448;   // 227 KB, the most one CTA can have on sm_100
 
-template <int D, bool BF16, bool SOFTCAP, bool B64>
+// SMs of the current device, looked up once per device (any host thread may be the first).
+static cudaError_t device_sm_count(int& sms) {
+  struct PerDevice {
+    std::once_flag once;
+    cudaError_t err = cudaSuccess;
+    int sms = 0;
+  };
+  static PerDevice per_device[kMaxDevices];
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  PerDevice& pd = per_device[dev];
+  std::call_once(pd.once, [&] { pd.err = cudaDeviceGetAttribute(&pd.sms, cudaDevAttrMultiProcessorCount, dev); });
+  sms = pd.sms;
+  return pd.err;
+}
+
+template <int D, bool BF16, bool SOFTCAP, bool B64, bool SPLIT>
 static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                                FwdParams p, cudaStream_t stream) {
-  auto kern = omni_fwd_ws_kernel<D, BF16, SOFTCAP, B64>;
-  const int smem = ws_smem_bytes<D>(p.nq, B64);
+  auto kern = omni_fwd_ws_kernel<D, BF16, SOFTCAP, B64, SPLIT>;
+  const int smem = ws_smem_bytes<D>(p.nq, B64, SPLIT);
   if (smem > kMaxSmemPerCta) return cudaErrorInvalidValue;   // the C-ABI layer refuses such lengths first
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -757,10 +888,13 @@ static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
     pd.err = cudaDeviceGetAttribute(&pd.num_sms, cudaDevAttrMultiProcessorCount, dev);
   });
   if (pd.err != cudaSuccess) return pd.err;
-  const int npairs = (p.nq + 1) / 2;
+  const int npairs = SPLIT ? p.nq : (p.nq + 1) / 2;
   const long long units = static_cast<long long>(npairs) * p.BH;
   p.num_units = static_cast<int>(units);
   const int grid = static_cast<int>(units < pd.num_sms ? units : pd.num_sms);
+  // A grid that holds every unit hands out nothing (the kernel's first units are its block numbers and the
+  // next of the fixed assignment does not exist), so the counter need not be cleared first.
+  if (units <= grid) p.unit_counter = nullptr;
   if (p.unit_counter != nullptr) {
     e = cudaMemsetAsync(p.unit_counter, 0, sizeof(int32_t), stream);
     if (e != cudaSuccess) return e;
@@ -769,16 +903,40 @@ static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
   return cudaGetLastError();
 }
 
+// Pairs of tiles keep K/V staging low but give a short batch few units: 8 heads of 2K tokens are 64 pairs for
+// 148 SMs, the longest of them 16 steps. There the split form pays, in which a unit is one tile and the two
+// softmax groups take its KV blocks in turn: twice the units, each with half the steps, twice the staging and a merge.
+// Pair against split form, us (head_dim 128 / 64, causal): 8 heads x 512 tokens 20.5 : 18.4 / 18.4 : 16.4; 8 x 2K
+// 43 : 31 / 39 : 27; 4 x 8K 127 : 78 / 115 : 68; 16 x 2K (0.86 pairs per SM) 43 : 37 / 39 : 31. Beyond one pair per SM
+// the pairs fill the chip: 12 x 4K (1.3) 74 : 72 / 66 : 59 but 32 x 1.5K (1.3) 39 : 47 / 35 : 39, 32 x 2K (1.7) 49 : 64 /
+// 43 : 51. Lists of at most 8 blocks leave too little to halve once the tiles outnumber the SMs: 32 x 1K 31 : 31 / 27 : 27,
+// with images 31 : 33 / 27 : 29.
+static bool use_split_units(int nq, int BH, int sms) {
+  const long long pairs = static_cast<long long>((nq + 1) / 2) * BH, tiles = static_cast<long long>(nq) * BH;
+  return pairs <= sms && (nq > 8 || tiles <= sms);
+}
+
+template <int D, bool BF16, bool SOFTCAP, bool B64>
+static cudaError_t launch_ws_s(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                               const FwdParams& p, cudaStream_t stream) {
+  int sms = 0;
+  const cudaError_t e = device_sm_count(sms);
+  if (e != cudaSuccess) return e;
+  const bool split = use_split_units(p.nq, p.BH, sms) && ws_smem_bytes<D>(p.nq, B64, true) <= kMaxSmemPerCta;
+  return split ? launch_ws_t<D, BF16, SOFTCAP, B64, true>(tmQ, tmK, tmV, p, stream)
+               : launch_ws_t<D, BF16, SOFTCAP, B64, false>(tmQ, tmK, tmV, p, stream);
+}
+
 template <int D, bool BF16>
 static cudaError_t launch_ws_d(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                                const FwdParams& p, cudaStream_t stream) {
   const bool cap = p.cap_out != 0.f;
   if (p.blk64) {
-    return cap ? launch_ws_t<D, BF16, true, true>(tmQ, tmK, tmV, p, stream)
-               : launch_ws_t<D, BF16, false, true>(tmQ, tmK, tmV, p, stream);
+    return cap ? launch_ws_s<D, BF16, true, true>(tmQ, tmK, tmV, p, stream)
+               : launch_ws_s<D, BF16, false, true>(tmQ, tmK, tmV, p, stream);
   }
-  return cap ? launch_ws_t<D, BF16, true, false>(tmQ, tmK, tmV, p, stream)
-             : launch_ws_t<D, BF16, false, false>(tmQ, tmK, tmV, p, stream);
+  return cap ? launch_ws_s<D, BF16, true, false>(tmQ, tmK, tmV, p, stream)
+             : launch_ws_s<D, BF16, false, false>(tmQ, tmK, tmV, p, stream);
 }
 
 // Longest sequence (in 128-row tiles) whose unit tables still fit beside the tiles in shared memory.
