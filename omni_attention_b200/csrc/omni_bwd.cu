@@ -62,54 +62,71 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// 1. Workspace: entry-code table and delta. Grid (nq, BH), 128 threads.
+// 1. Workspace: entry-code table and delta. Grid (nq, BH), 160 threads: warps 0-3 compute delta of 32 rows
+// each, warp 4 resolves the Q block's list. Bound by the two 16-bit tensors read once, and for short batches by
+// load latency alone, so each warp has kBatch loads of 16 bytes per lane and tensor in flight, several rows at a
+// time (one row at a time, 4 bytes per lane: 25 us whatever the length below 2K tokens).
 // ---------------------------------------------------------------------------------------------
+constexpr int kPrepThreads = 160;
 template <int D, bool BF16>
-__global__ void __launch_bounds__(128) omni_bwd_prep_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(kPrepThreads) omni_bwd_prep_kernel(const BwdParams p) {
   const int tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
   const int qb = blockIdx.x;
   const int bh = blockIdx.y;
   const int nq = p.f.nq;
 
   uint32_t* codes = p.codes + (static_cast<long long>(bh) * nq + qb) * nq;
-  for (int i = tid; i < nq; i += 128) codes[i] = 0u;
-  __syncthreads();
-  const long long list_base = (static_cast<long long>(bh) * nq + qb) * p.f.max_blocks;
-  int n_list = __ldg(p.f.kv_num_blocks + static_cast<long long>(bh) * nq + qb);
-  n_list = max(0, min(n_list, p.f.max_blocks));
-  if (tid < 32) {   // one warp walks the list in order; a block listed twice resolves as in the forward
-    for (int i0 = 0; i0 < n_list; i0 += 32) {
-      const int i = i0 + tid;
+  if (warp == 4) {
+    for (int i = lane; i < nq; i += 32) codes[i] = 0u;
+    __syncwarp();
+    const long long list_base = (static_cast<long long>(bh) * nq + qb) * p.f.max_blocks;
+    int n_list = __ldg(p.f.kv_num_blocks + static_cast<long long>(bh) * nq + qb);
+    n_list = max(0, min(n_list, p.f.max_blocks));
+    for (int i0 = 0; i0 < n_list; i0 += 32) {   // in list order; a block listed twice resolves as in the forward
+      const int i = i0 + lane;
       int kvb = -1;
       uint32_t code = 0u;
       if (i < n_list) code = resolve_entry(p.f, list_base, i, qb, kvb);
       table_put(codes, code != 0u ? kvb : -1, code);
     }
+    return;
   }
 
-  // delta: one warp per row at a time, D / 32 elements per lane
-  const int warp = tid >> 5, lane = tid & 31;
-  constexpr int kWords = D / 64;   // 32-bit words (2 elements) per lane
-  for (int rr = 0; rr < 32; ++rr) {
-    if (qb * kBlock + warp * 32 + rr >= p.f.N) break;   // the last tile of an unpadded tensor
-    const long long row = static_cast<long long>(bh) * p.f.N + qb * kBlock + warp * 32 + rr;
-    // rows are d_real elements long (head_dim 32 runs on the 64-wide instantiation: the upper lanes idle)
-    const long long pitch = static_cast<long long>(p.f.d_real) * 2;
-    const uint32_t* po = reinterpret_cast<const uint32_t*>(static_cast<const char*>(p.o) + row * pitch) + lane * kWords;
-    const uint32_t* pd = reinterpret_cast<const uint32_t*>(static_cast<const char*>(p.d_o) + row * pitch) + lane * kWords;
-    float acc = 0.f;
-    if (lane * kWords * 2 < p.f.d_real) {
+  constexpr int kLanes = D / 8;               // lanes per row, 16 bytes each
+  constexpr int kRowsAtOnce = 32 / kLanes;
+  constexpr int kBatch = 4;
+  const int sub = lane / kLanes, col = (lane % kLanes) * 8;
+  const bool in_row = col < p.f.d_real;       // head_dim 32 on the 64-wide instantiation: half the lanes idle
+  const long long pitch = static_cast<long long>(p.f.d_real) * 2;
+  const long long head = static_cast<long long>(bh) * p.f.N;
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += kRowsAtOnce * kBatch) {
+    uint4 a[kBatch], b[kBatch];
 #pragma unroll
-      for (int w = 0; w < kWords; ++w) {
-        const float2 a = unpack2<BF16>(__ldg(po + w));
-        const float2 b = unpack2<BF16>(__ldg(pd + w));
-        acc = fmaf(a.x, b.x, acc);
-        acc = fmaf(a.y, b.y, acc);
+    for (int i = 0; i < kBatch; ++i) {
+      const int q_abs = qb * kBlock + 32 * warp + r0 + kRowsAtOnce * i + sub;
+      a[i] = b[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (in_row && q_abs < p.f.N) {   // the last tile of an unpadded tensor ends inside
+        a[i] = __ldg(reinterpret_cast<const uint4*>(static_cast<const char*>(p.o) + (head + q_abs) * pitch + 2 * col));
+        b[i] = __ldg(reinterpret_cast<const uint4*>(static_cast<const char*>(p.d_o) + (head + q_abs) * pitch + 2 * col));
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-    if (lane == 0) p.delta[row] = acc;
+    for (int i = 0; i < kBatch; ++i) {
+      const int q_abs = qb * kBlock + 32 * warp + r0 + kRowsAtOnce * i + sub;
+      const uint32_t wa[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, wb[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+      float acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float2 x = unpack2<BF16>(wa[w]), y = unpack2<BF16>(wb[w]);
+        acc = fmaf(x.x, y.x, acc);
+        acc = fmaf(x.y, y.y, acc);
+      }
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+      if (lane % kLanes == 0 && q_abs < p.f.N) p.delta[head + q_abs] = acc;
+    }
   }
 }
 
@@ -886,7 +903,7 @@ static cudaError_t launch_bwd_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, 
   e = ensure_smem_attr(dq, DqCfg<D>::kSmemBytes, attr_dq);
   if (e != cudaSuccess) return e;
   const dim3 grid(p.f.nq, p.f.BH);
-  omni_bwd_prep_kernel<D, BF16><<<grid, 128, 0, stream>>>(p);
+  omni_bwd_prep_kernel<D, BF16><<<grid, kPrepThreads, 0, stream>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const unsigned ctas = static_cast<unsigned>(p.f.nq) * static_cast<unsigned>(p.f.BH);
