@@ -40,11 +40,22 @@ struct BwdCfg {
   static constexpr int kChunks = D / 64;
   static constexpr int kChunkBytes = kBlock * 128;
   static constexpr int kTmemCols = 512;
-  static constexpr int kVecBytes = 2 * 2 * kBlock * 4;   // LSE and delta of a Q block, two stages
-  static constexpr int kBitsBytes = kBlock * 16;          // one bit-packed partial tile
+  // dK/dV kernel: whether S^T has two regions of TMEM (free next to dV and dK at D = 64) and is issued a visit
+  // ahead, and the stages of Q, LSE and delta that this takes
+  static constexpr bool kAhead = (D == 64);
+  static constexpr int kQStages = kAhead ? 3 : 2;
+  static constexpr int kVecBytes = 2 * kQStages * kBlock * 4;   // LSE and delta of a Q block
+  static constexpr int kBitsBytes = 2 * kBlock * 16;      // bit-packed partial tiles of two visits
   static constexpr int kListBytes = kMaxKvBlocks * 4 + kMaxKvBlocks * 2 + 16;   // codes, visit list, its length
-  static constexpr int kSmemBytes = 6 * kTileBytes + kVecBytes + kBitsBytes + kListBytes + 256 + 1024;
+  static constexpr int kSmemBytes = (4 + kQStages) * kTileBytes + kVecBytes + kBitsBytes + kListBytes + 256 + 1024;
 };
+
+// Of every eight element pairs, this many take their exponentials from the FMA pipe (exp2_fma2): the two halves of
+// the per-element work alternate, so while E1 runs the MUFU unit is what it waits for (1 024 cycles a visit). dK/dV
+// kernel 956 -> 942 / 934 / 938 us with 1 / 2 / 3 of eight (32 heads x 8K tokens, D = 128) and 234 -> 227 / 225 / 224
+// (32 x 4K, D = 64); dQ kernel 710 -> 704 / 698 / 700 and 172 -> 170 / 167 / 166.
+// Not with a soft-cap, whose own polynomial already fills that pipe (dQ kernel of 16 heads x 1.5K tokens 34 -> 36 us).
+constexpr int kBwdPolyOf8 = 2;
 
 constexpr int kBwdComputeThreads = 256;
 constexpr int kBwdThreads = kBwdComputeThreads + 64;
@@ -281,19 +292,25 @@ __device__ __forceinline__ float lse_to_log2(float lse) {
 //              [0,64) and [64,128) of the visited Q block)
 //   warp  8    first lane issues every tcgen05.mma
 //   warp  9    first lane issues the TMA loads
-// TMEM: S^T [0,128), dP^T [128,256), dV [256,256+D), dK [384,384+D). P^T (16-bit) goes over S^T and
-// dS^T over dP^T, each thread writing only columns it has read itself.
+// TMEM, D = 128: S^T [0,128), dP^T [128,256), dV [256,384), dK [384,512); P^T (16-bit) goes over S^T and
+// dS^T over dP^T. D = 64: two regions of S^T [0,256), dP^T [256,384), dV [384,448), dK [448,512); P^T and dS^T
+// both go over S^T. Each thread writes only columns it has read itself.
 //
 // The per-element work is split in two so that the tensor pipe always has something to do:
 //   E1(i): P^T  = exp2(S^T * c - LSE)        needs S^T(i)          -> feeds dV(i)
 //   E2(i): dS^T = P^T * (dP^T - delta)       needs dP^T(i), E1(i)  -> feeds dK(i)
-// and the MMAs of consecutive visits are interleaved in the order
+// and the MMAs of consecutive visits are interleaved, at D = 128 in the order
 //   dV(i), S^T(i+1) | dK(i), dP^T(i+1)
 // The first pair is issued when P^T(i) is there and runs under E2(i), the second when dS^T(i) is there and
 // runs under E1(i+1): each region is overwritten by the MMA right behind the one that read it, so neither
 // half of the per-element work waits for more than the pair in front of it. (With the regions alternating,
 // S^T(i+1) over dP^T(i) and so only after E2(i), the chain S^T - E1 - E2 of a visit could not overlap the next
-// one's: kernel 1055 against 949 us for 32 heads x 8K tokens at D = 128, bits equal.)
+// one's: kernel 1055 against 949 us for 32 heads x 8K tokens at D = 128, bits equal.) The 32 MMAs of a visit are
+// then 2 560 of its about 3 000 cycles (80 each: their operands and the TMA writes share the shared-memory port).
+// D = 64 needs half the MMAs and is bound by the per-element work; its second region of S^T lets the scores run a
+// visit ahead, so that E1(i+1) starts as soon as E2(i) ends:
+//   dV(i) | dP^T(i+1), dK(i), S^T(i+2)
+// (32 heads x 4K tokens: 230 -> 211 us together with the vectors staged by the producer warp and kBwdPolyOf8.)
 // ---------------------------------------------------------------------------------------------
 template <int D, bool BF16, bool SOFTCAP>
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -307,30 +324,32 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   const uint32_t sK = smem_u32(smem);
   const uint32_t sV = sK + Cfg::kTileBytes;
-  const uint32_t sQ = sV + Cfg::kTileBytes;            // two stages
-  const uint32_t sdO = sQ + 2 * Cfg::kTileBytes;       // two stages
-  // LSE (+inf for a dead row) and delta of the visited Q block as loaded, two stages
-  float* lse_s = reinterpret_cast<float*>(smem + 6 * Cfg::kTileBytes);   // [2][128]
-  float* delta_s = lse_s + 2 * kBlock;                                    // [2][128]
-  uint32_t* bits_s = reinterpret_cast<uint32_t*>(delta_s + 2 * kBlock);   // [128][4]
-  uint32_t* code_s = bits_s + kBlock * 4;                                   // [kMaxKvBlocks]
+  const uint32_t sQ = sV + Cfg::kTileBytes;                  // kQStages
+  const uint32_t sdO = sQ + Cfg::kQStages * Cfg::kTileBytes;  // two stages
+  // -LSE * log2(e) (-inf for a dead row) and -delta of the visited Q block, kQStages
+  float* lse_s = reinterpret_cast<float*>(smem + (4 + Cfg::kQStages) * Cfg::kTileBytes);   // [kQStages][128]
+  float* delta_s = lse_s + Cfg::kQStages * kBlock;                                         // [kQStages][128]
+  uint32_t* bits_s = reinterpret_cast<uint32_t*>(delta_s + Cfg::kQStages * kBlock);        // [2][128][4]
+  uint32_t* code_s = bits_s + 2 * kBlock * 4;                                // [kMaxKvBlocks]
   uint16_t* vis_s = reinterpret_cast<uint16_t*>(code_s + kMaxKvBlocks);      // [kMaxKvBlocks]
   int* n_vis_s = reinterpret_cast<int*>(vis_s + kMaxKvBlocks);
   uint64_t* bars = reinterpret_cast<uint64_t*>(n_vis_s + 4);
   const uint32_t bar_kv = smem_u32(bars + 0);       // K, V landed
-  const uint32_t bar_q = smem_u32(bars + 1);        // [2] Q stage landed
-  const uint32_t bar_do = smem_u32(bars + 3);       // [2] dO stage landed
-  const uint32_t bar_s = smem_u32(bars + 5);        // S^T of the visit complete
-  const uint32_t bar_dp = smem_u32(bars + 6);       // dP^T of the visit complete
-  const uint32_t bar_p = smem_u32(bars + 7);        // P^T stored (256 arrivals)
-  const uint32_t bar_ds = smem_u32(bars + 8);       // dS^T stored (256 arrivals)
-  const uint32_t bar_dvdone = smem_u32(bars + 9);   // [2] dV MMAs of the visit in this stage complete: dO stage free
-  const uint32_t bar_dkdone = smem_u32(bars + 11);  // [2] dK MMAs complete: Q stage free
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  const uint32_t bar_q = smem_u32(bars + 1);        // [3] Q stage landed
+  const uint32_t bar_do = smem_u32(bars + 4);       // [2] dO stage landed
+  const uint32_t bar_s = smem_u32(bars + 6);        // [2] S^T of a visit complete (by visit parity)
+  const uint32_t bar_dp = smem_u32(bars + 8);       // dP^T of the visit complete
+  const uint32_t bar_p = smem_u32(bars + 9);        // P^T stored (256 arrivals)
+  const uint32_t bar_ds = smem_u32(bars + 10);      // dS^T stored (256 arrivals)
+  const uint32_t bar_dvdone = smem_u32(bars + 11);  // [2] dV MMAs of the visit in this stage complete: dO stage free
+  const uint32_t bar_dkdone = smem_u32(bars + 13);  // [3] dK MMAs complete: Q, LSE and delta stage free
+  const uint32_t bar_vec = smem_u32(bars + 16);     // [3] LSE / delta of the visit in this stage written (32 arrivals)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
+  const int lane = tid & 31;
   const bool compute = tid < kBwdComputeThreads;
   const int half = (tid >> 7) & 1;  // which 64 query columns of the tile this thread works on
   const int t = tid & 127;          // key row of the tile = TMEM lane
@@ -340,13 +359,16 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (tid == 0) {
     mbar_init(bar_kv, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < 3; ++s) {
       mbar_init(bar_q + 8 * s, 1);
+      mbar_init(bar_dkdone + 8 * s, 1);
+      mbar_init(bar_vec + 8 * s, 32);
+    }
+    for (int s = 0; s < 2; ++s) {
       mbar_init(bar_do + 8 * s, 1);
       mbar_init(bar_dvdone + 8 * s, 1);
-      mbar_init(bar_dkdone + 8 * s, 1);
+      mbar_init(bar_s + 8 * s, 1);
     }
-    mbar_init(bar_s, 1);
     mbar_init(bar_dp, 1);
     mbar_init(bar_p, kBwdComputeThreads);
     mbar_init(bar_ds, kBwdComputeThreads);
@@ -367,10 +389,13 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const uint32_t tS = tmem_base;
-  const uint32_t tdP = tmem_base + 128;
-  const uint32_t tdV = tmem_base + 256;
-  const uint32_t tdK = tmem_base + 384;
+  auto region_s = [&](int i) { return tmem_base + (Cfg::kAhead ? 128u * static_cast<uint32_t>(i & 1) : 0u); };
+  const uint32_t tdP = tmem_base + (Cfg::kAhead ? 256 : 128);
+  const uint32_t tdV = tmem_base + 512 - 2 * D;
+  const uint32_t tdK = tmem_base + 512 - D;
+  // where dS^T goes, from a thread's 64 columns on: behind P^T over S^T, or over dP^T
+  auto region_ds = [&](int i) { return Cfg::kAhead ? region_s(i) : tdP; };
+  constexpr uint32_t kDsOff = Cfg::kAhead ? 32 : 0;
   constexpr int fmt = BF16 ? 1 : 0;
   constexpr uint32_t idesc_ss = umma_idesc_f16(128, 128, fmt, 0);
   constexpr uint32_t idesc_ts = umma_idesc_f16(128, D, fmt, 1);
@@ -379,58 +404,97 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   // column kvb of this head's code table: which Q blocks visit this KV block, and how
   const int n_vis = bwd_build_visit_list(p.codes + static_cast<long long>(bh) * nq * nq + kvb, nq, nq, code_s, vis_s,
                                          n_vis_s);
-  auto stage_vectors = [&](int qb, int stage) {   // threads 0-127
-    const int q_abs = qb * kBlock + tid;
-    const long long row = row0 + q_abs;
+  // What the compute warps need of query row q_abs: -LSE * log2(e), -inf for a row beyond the sequence or one
+  // that attended nothing, and -delta.
+  auto load_vectors = [&](int q_abs, float& neg_lse2, float& neg_delta) {
     const bool live = q_abs < p.f.seqlen_orig;
-    const float l = live ? __ldg(p.lse + row) : INFINITY;
-    lse_s[stage * kBlock + tid] = l == -INFINITY ? INFINITY : l;   // a row that attended nothing is dead too
-    delta_s[stage * kBlock + tid] = live ? __ldg(p.delta + row) : 0.f;
+    neg_lse2 = live ? -lse_to_log2(__ldg(p.lse + row0 + q_abs)) : -INFINITY;
+    neg_delta = live ? -__ldg(p.delta + row0 + q_abs) : 0.f;
   };
-  if (tid < kBlock) {
-    if (n_vis > 0) stage_vectors(vis_s[0], 0);
-    if (n_vis > 1) stage_vectors(vis_s[1], 1);
+  if constexpr (!Cfg::kAhead) {
+    if (tid < kBlock) {
+      for (int i = 0; i < 2 && i < n_vis; ++i) {
+        load_vectors(static_cast<int>(vis_s[i]) * kBlock + tid, lse_s[i * kBlock + tid], delta_s[i * kBlock + tid]);
+      }
+    }
+    __syncthreads();   // the vectors are read by every compute thread
   }
-  __syncthreads();   // the LSE / delta vectors are read by every compute thread
 
-  if (warp == kBwdProducerWarp && elect_one()) {
+  if (warp == kBwdProducerWarp && (Cfg::kAhead || elect_one())) {
     // =========================== TMA producer ====================================================
-    if (n_vis > 0) {
+    // With S^T issued ahead, the whole warp runs this loop: one elected lane issues the copies and all stage the
+    // LSE / delta vectors (rows of unpadded tensors have no alignment that a bulk copy could use) in the form the
+    // compute warps need them in. A stage of Q and of the vectors is free when dK of its last visit, which was
+    // issued after every compute thread had stored dS^T, is complete. Without (D = 128) one lane issues the
+    // copies and the compute warps stage the vectors: there the loop waits on the tensor pipe anyway, and the
+    // vectors in this warp made the kernel slower (984 against 945 us; at D = 64 223 against 233).
+    const bool leader = Cfg::kAhead ? elect_one() : true;
+    auto wait = [&](uint32_t bar, uint32_t parity, int where) {
+      if constexpr (Cfg::kAhead) {
+        mbar_wait_warp(bar, parity, abort_flag, p.f.status, where);
+      } else {
+        mbar_wait(bar, parity, abort_flag, p.f.status, where);
+      }
+    };
+    if (n_vis > 0 && leader) {
       mbar_expect_tx(bar_kv, 2 * Cfg::kTileBytes);
       const int y = kvb * kBlock;
       bwd_load_tile<D>(sK, &tmK, bar_kv, y, bh);
       bwd_load_tile<D>(sV, &tmV, bar_kv, y, bh);
     }
-    for (int i = 0; i < n_vis; ++i) {
-      const int stage = i & 1;
+    auto load_q = [&](int i) {
+      const int stage = i % Cfg::kQStages;
       const int y = static_cast<int>(vis_s[i]) * kBlock;
-      const uint32_t prev = static_cast<uint32_t>(((i >> 1) - 1) & 1);   // parity of the stage's previous use
-      auto load_q = [&] {
-        if (i >= 2) mbar_wait(bar_dkdone + 8 * stage, prev, abort_flag, p.f.status, 55);
+      float vl[4], vd[4];   // in flight while the stage is waited for
+      if constexpr (Cfg::kAhead) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) load_vectors(y + 32 * j + lane, vl[j], vd[j]);
+      }
+      if (i >= Cfg::kQStages) {
+        wait(bar_dkdone + 8 * stage, static_cast<uint32_t>((i / Cfg::kQStages - 1) & 1), 55);
+      }
+      if (leader) {
         mbar_expect_tx(bar_q + 8 * stage, Cfg::kTileBytes);
         bwd_load_tile<D>(sQ + stage * Cfg::kTileBytes, &tmQ, bar_q + 8 * stage, y, bh);
-      };
-      auto load_do = [&] {
-        if (i >= 2) mbar_wait(bar_dvdone + 8 * stage, prev, abort_flag, p.f.status, 56);
+      }
+      if constexpr (Cfg::kAhead) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          lse_s[stage * kBlock + 32 * j + lane] = vl[j];
+          delta_s[stage * kBlock + 32 * j + lane] = vd[j];
+        }
+        mbar_arrive(bar_vec + 8 * stage);
+      }
+    };
+    auto load_do = [&](int i) {
+      const int stage = i & 1;
+      if (i >= 2) wait(bar_dvdone + 8 * stage, static_cast<uint32_t>(((i >> 1) - 1) & 1), 56);
+      if (leader) {
         mbar_expect_tx(bar_do + 8 * stage, Cfg::kTileBytes);
-        bwd_load_tile<D>(sdO + stage * Cfg::kTileBytes, &tmdO, bar_do + 8 * stage, y, bh);
-      };
-      if (i < 2) {   // both stages are empty: what the visit needs first
-        load_q();
-        load_do();
-      } else {       // in the order in which the stages come free
-        load_do();
-        load_q();
+        bwd_load_tile<D>(sdO + stage * Cfg::kTileBytes, &tmdO, bar_do + 8 * stage, static_cast<int>(vis_s[i]) * kBlock, bh);
+      }
+    };
+    if (Cfg::kAhead && n_vis > 0) load_q(0);
+    for (int i = 0; i < n_vis; ++i) {   // in the order in which the stages come free
+      if constexpr (Cfg::kAhead) {
+        load_do(i);
+        if (i + 1 < n_vis) load_q(i + 1);
+      } else if (i < 2) {   // both stages are empty: what the visit needs first
+        load_q(i);
+        load_do(i);
+      } else {
+        load_do(i);
+        load_q(i);
       }
     }
   } else if (warp == kBwdIssuerWarp && elect_one()) {
     // =========================== MMA issuer ======================================================
     auto issue_s = [&](int i) {    // S^T(i) = K Q(i)^T
-      const int stage = i & 1;
-      mbar_wait(bar_q + 8 * stage, static_cast<uint32_t>((i >> 1) & 1), abort_flag, p.f.status, 51);
+      const int stage = i % Cfg::kQStages;
+      mbar_wait(bar_q + 8 * stage, static_cast<uint32_t>((i / Cfg::kQStages) & 1), abort_flag, p.f.status, 51);
       tc_fence_after();
-      bwd_mma_ss<D>(tS, sK, sQ + stage * Cfg::kTileBytes, idesc_ss);
-      tc_commit(bar_s);
+      bwd_mma_ss<D>(region_s(i), sK, sQ + stage * Cfg::kTileBytes, idesc_ss);
+      tc_commit(bar_s + 8 * (i & 1));
     };
     auto issue_dp = [&](int i) {   // dP^T(i) = V dO(i)^T
       const int stage = i & 1;
@@ -439,10 +503,16 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       bwd_mma_ss<D>(tdP, sV, sdO + stage * Cfg::kTileBytes, idesc_ss);
       tc_commit(bar_dp);
     };
+    auto issue_dk = [&](int i) {   // dK += dS^T(i) Q(i)
+      const int stage = i % Cfg::kQStages;
+      bwd_mma_ts_split<D>(tdK, region_ds(i), kDsOff, sQ + stage * Cfg::kTileBytes, idesc_ts, i > 0);
+      tc_commit(bar_dkdone + 8 * stage);
+    };
     if (n_vis > 0) {
       mbar_wait(bar_kv, 0, abort_flag, p.f.status, 50);
       issue_s(0);
       issue_dp(0);
+      if (Cfg::kAhead && n_vis > 1) issue_s(1);
     }
     for (int i = 0; i < n_vis; ++i) {
       const int stage = i & 1;
@@ -450,42 +520,47 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // E1(i) has read S^T(i) and stored P^T(i) over it
       mbar_wait(bar_p, ph, abort_flag, p.f.status, 58);
       tc_fence_after();
-      bwd_mma_ts_split<D>(tdV, tS, 0, sdO + stage * Cfg::kTileBytes, idesc_ts, i > 0);    // dV += P^T(i) dO(i)
+      bwd_mma_ts_split<D>(tdV, region_s(i), 0, sdO + stage * Cfg::kTileBytes, idesc_ts, i > 0);    // dV += P^T(i) dO(i)
       tc_commit(bar_dvdone + 8 * stage);
-      if (i + 1 < n_vis) issue_s(i + 1);   // over P^T(i), which the MMAs just issued read first
-      // E2(i) has read dP^T(i) and stored dS^T(i) over it
+      if (!Cfg::kAhead && i + 1 < n_vis) issue_s(i + 1);   // over P^T(i), which the MMAs just issued read first
+      // E2(i) has read dP^T(i) and stored dS^T(i)
       mbar_wait(bar_ds, ph, abort_flag, p.f.status, 57);
       tc_fence_after();
-      bwd_mma_ts_split<D>(tdK, tdP, 0, sQ + stage * Cfg::kTileBytes, idesc_ts, i > 0);    // dK += dS^T(i) Q(i)
-      tc_commit(bar_dkdone + 8 * stage);
-      if (i + 1 < n_vis) issue_dp(i + 1);
+      if constexpr (Cfg::kAhead) {
+        if (i + 1 < n_vis) issue_dp(i + 1);   // first: E2(i + 1) waits for it
+        issue_dk(i);
+        if (i + 2 < n_vis) issue_s(i + 2);    // over P^T(i) and dS^T(i)
+      } else {
+        issue_dk(i);
+        if (i + 1 < n_vis) issue_dp(i + 1);   // over dS^T(i)
+      }
     }
     if (n_vis > 0) {
       const int last = n_vis - 1;
       // keep this thread alive until every MMA has retired
-      mbar_wait(bar_dkdone + 8 * (last & 1), static_cast<uint32_t>((last >> 1) & 1), abort_flag, p.f.status, 59);
+      mbar_wait(bar_dkdone + 8 * (last % Cfg::kQStages), static_cast<uint32_t>((last / Cfg::kQStages) & 1), abort_flag,
+                p.f.status, 59);
     }
   } else if (compute) {
     // =========================== per-element work ================================================
     const int k_abs = kvb * kBlock + t;
     const bool key_live = k_abs < p.f.seqlen_orig;
     const float2 c2 = make_float2(p.f.scale_log2, p.f.scale_log2);
+    int next_qb = n_vis > 0 ? vis_s[0] : 0;   // looked up one visit ahead
+    uint32_t next_code = code_s[next_qb];
     for (int i = 0; i < n_vis; ++i) {
-      const int stage = i & 1;
+      const int stage = i % Cfg::kQStages;
       const uint32_t ph = static_cast<uint32_t>(i & 1);
-      const int qb = vis_s[i];
-      const uint32_t code = code_s[qb];
-      const uint32_t my_s = tS + lane_base + 64 * half;
+      const int qb = next_qb;
+      const uint32_t code = next_code;
+      const uint32_t my_s = region_s(i) + lane_base + 64 * half;
       const uint32_t my_dp = tdP + lane_base + 64 * half;
-      // LSE / delta of the visit after next: the global loads are issued here and land in shared
-      // memory at the end of this visit (stored as loaded), so their latency is off everybody's path
-      float next_lse = INFINITY, next_delta = 0.f;
-      if (tid < kBlock && i + 2 < n_vis) {
-        const int q_abs = static_cast<int>(vis_s[i + 2]) * kBlock + tid;
-        if (q_abs < p.f.seqlen_orig) {
-          next_lse = __ldg(p.lse + row0 + q_abs);
-          next_delta = __ldg(p.delta + row0 + q_abs);
-        }
+      const uint32_t my_ds = region_ds(i) + kDsOff + lane_base + 64 * half;
+      // D = 128: the vectors of the visit after next, loaded here and stored at the end of this visit, so that
+      // their latency is off everybody's path
+      float next_lse = -INFINITY, next_delta = 0.f;
+      if (!Cfg::kAhead && tid < kBlock && i + 2 < n_vis) {
+        load_vectors(static_cast<int>(vis_s[i + 2]) * kBlock + tid, next_lse, next_delta);
       }
 
       // Allow-bits of this thread's key over its 64 query rows of the block (bit r of word w = query
@@ -493,10 +568,12 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t type = code & kCodeTypeMask;
       uint32_t allow[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
       if (type == kTypePartial) {   // uniform over the compute threads
+        // (the buffer's last use was two visits ago: dP^T of the last visit came after every dS^T of that one)
+        uint32_t* bits = bits_s + (i & 1) * kBlock * 4;
         if (tid < kBlock) {
           uint32_t rowbits[4];
           load_partial_row(p.f, code >> 3, tid, rowbits);   // row tid of the tile = query row tid
-          *reinterpret_cast<uint4*>(bits_s + 4 * tid) = make_uint4(rowbits[0], rowbits[1], rowbits[2], rowbits[3]);
+          *reinterpret_cast<uint4*>(bits + 4 * tid) = make_uint4(rowbits[0], rowbits[1], rowbits[2], rowbits[3]);
         }
         named_barrier_sync(1, kBwdComputeThreads);
 #pragma unroll
@@ -504,7 +581,7 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           uint32_t acc = 0u;
 #pragma unroll
           for (int r = 0; r < 32; ++r) {
-            acc |= ((bits_s[4 * (64 * half + 32 * w + r) + (t >> 5)] >> (t & 31)) & 1u) << r;
+            acc |= ((bits[4 * (64 * half + 32 * w + r) + (t >> 5)] >> (t & 31)) & 1u) << r;
           }
           allow[w] = acc;
         }
@@ -531,7 +608,10 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const float* lse_c = lse_s + stage * kBlock + 64 * half;
       const float* del_c = delta_s + stage * kBlock + 64 * half;
       float pf[64];      // the unrounded probabilities (times the soft-cap slope, if any), kept for E2
-      mbar_wait_warp(bar_s, ph, abort_flag, p.f.status, 52);
+      if constexpr (Cfg::kAhead) {
+        mbar_wait_warp(bar_vec + 8 * stage, static_cast<uint32_t>((i / Cfg::kQStages) & 1), abort_flag, p.f.status, 49);
+      }
+      mbar_wait_warp(bar_s + 8 * (i & 1), static_cast<uint32_t>((i >> 1) & 1), abort_flag, p.f.status, 52);
       tc_fence_after();
       auto e1 = [&](auto masked_c) {
         constexpr bool kMasked = decltype(masked_c)::value;
@@ -546,13 +626,12 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const uint32_t aw = allow[c];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            const float2 nl = __fmul2_rn(*reinterpret_cast<const float2*>(lse_c + 32 * c + 2 * j),
-                                         make_float2(-1.4426950408889634f, -1.4426950408889634f));   // +inf (dead row) -> -inf
+            const float2 nl = *reinterpret_cast<const float2*>(lse_c + 32 * c + 2 * j);
             float2 sc = make_float2(__uint_as_float(rs[2 * j]), __uint_as_float(rs[2 * j + 1]));
             float2 slope = make_float2(1.f, 1.f);
             if constexpr (SOFTCAP) slope = bwd_soft_cap(sc, p.f.cap_in, p.f.cap_out);
             const float2 x = __ffma2_rn(sc, c2, nl);
-            float2 pr = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+            float2 pr = j % 8 < (SOFTCAP ? 0 : kBwdPolyOf8) ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
             if constexpr (kMasked) {
               pr.x = ((aw >> (2 * j)) & 1u) ? pr.x : 0.f;
               pr.y = ((aw >> (2 * j + 1)) & 1u) ? pr.y : 0.f;
@@ -575,6 +654,11 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_before();
       mbar_arrive(bar_p);
 
+      if (i + 1 < n_vis) {
+        next_qb = vis_s[i + 1];
+        next_code = code_s[next_qb];
+      }
+
       // ---- E2: dS^T ------------------------------------------------------------------------------
       mbar_wait_warp(bar_dp, ph, abort_flag, p.f.status, 53);
       tc_fence_after();
@@ -588,30 +672,34 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         uint32_t dd[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float2 dl = *reinterpret_cast<const float2*>(del_c + 32 * c + 2 * j);
+          const float2 nd = *reinterpret_cast<const float2*>(del_c + 32 * c + 2 * j);
           const float2 ds = __fmul2_rn(make_float2(pf[32 * c + 2 * j], pf[32 * c + 2 * j + 1]),
                                        __fadd2_rn(make_float2(__uint_as_float(rd[2 * j]), __uint_as_float(rd[2 * j + 1])),
-                                                  make_float2(-dl.x, -dl.y)));
+                                                  nd));
           dd[j] = pack2<BF16>(ds.x, ds.y);
         }
-        // dS^T over this thread's dP^T columns [0,32) of its half (all read above)
-        tmem_st16(my_dp + 16 * c, dd);
+        // over columns of its half that this thread has read
+        tmem_st16(my_ds + 16 * c, dd);
       }
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(bar_ds);
-
-      // the vectors (and the partial-mask bits) of this visit are free once every compute thread is
-      // through E2
-      named_barrier_sync(2, kBwdComputeThreads);
-      if (tid < kBlock && i + 2 < n_vis) {
-        lse_s[stage * kBlock + tid] = next_lse == -INFINITY ? INFINITY : next_lse;
-        delta_s[stage * kBlock + tid] = next_delta;
+      if constexpr (!Cfg::kAhead) {   // this visit's vectors are free once every compute thread is through E2
+        named_barrier_sync(2, kBwdComputeThreads);
+        if (tid < kBlock && i + 2 < n_vis) {
+          lse_s[stage * kBlock + tid] = next_lse;
+          delta_s[stage * kBlock + tid] = next_delta;
+        }
       }
     }
     if (n_vis > 0) {
       const int last = n_vis - 1;
-      mbar_wait_warp(bar_dkdone + 8 * (last & 1), static_cast<uint32_t>((last >> 1) & 1), abort_flag, p.f.status, 54);
+      if (half == 0) {   // dV is complete before dK
+        mbar_wait_warp(bar_dvdone + 8 * (last & 1), static_cast<uint32_t>((last >> 1) & 1), abort_flag, p.f.status, 54);
+      } else {
+        mbar_wait_warp(bar_dkdone + 8 * (last % Cfg::kQStages), static_cast<uint32_t>((last / Cfg::kQStages) & 1), abort_flag,
+                       p.f.status, 54);
+      }
       tc_fence_after();
     }
     const long long out_row = row0 + k_abs;
@@ -833,7 +921,7 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             float2 slope = make_float2(1.f, 1.f);
             if constexpr (SOFTCAP) slope = bwd_soft_cap(sc, p.f.cap_in, p.f.cap_out);
             const float2 x = __ffma2_rn(sc, c2, nl2);
-            float2 pr = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+            float2 pr = j % 8 < (SOFTCAP ? 0 : kBwdPolyOf8) ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
             if constexpr (SOFTCAP) pr = __fmul2_rn(pr, slope);
             if constexpr (kMasked) {
               pr.x = ((aw >> (2 * j)) & 1u) ? pr.x : 0.f;

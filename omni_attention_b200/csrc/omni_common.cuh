@@ -238,6 +238,17 @@ __device__ __forceinline__ void load_partial_row(const FwdParams& p, uint32_t pi
   }
 }
 
+// One word of it (keys 32 * w .. 32 * w + 31).
+__device__ __forceinline__ uint32_t load_partial_word(const FwdParams& p, uint32_t pidx, int r, int w) {
+  const size_t row = static_cast<size_t>(pidx) * kBlock + r;
+  if (p.partial_bits != nullptr) return __ldg(p.partial_bits + row * 4 + w);
+  const uint4* src = reinterpret_cast<const uint4*>(p.partial_bool + row * kBlock) + 2 * w;
+  const uint4 a = __ldg(src), b = __ldg(src + 1);
+  return bytes_to_nibble(a.x) | (bytes_to_nibble(a.y) << 4) | (bytes_to_nibble(a.z) << 8) | (bytes_to_nibble(a.w) << 12) |
+         (bytes_to_nibble(b.x) << 16) | (bytes_to_nibble(b.y) << 20) | (bytes_to_nibble(b.z) << 24) |
+         (bytes_to_nibble(b.w) << 28);
+}
+
 // Allow-bits of row r for a diagonal CAUSAL tile: column c allowed iff c <= r.
 __device__ __forceinline__ void causal_row(int r, uint32_t (&allow)[4]) {
 #pragma unroll
@@ -490,6 +501,26 @@ constexpr float kExp2C1 = 0.6932610273361206f;
 constexpr float kExp2C2 = 0.24261116981506348f;
 constexpr float kExp2C3 = 0.0551714189350605f;
 constexpr float kRoundMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to the nearest integer
+
+// 2^x of two values on the FMA pipe to the accuracy of ex2.approx (largest relative error 1.7e-7; the MUFU unit's is
+// stated as 2^-22): n = round(x), a minimax polynomial of degree 5 with constant term 1 for 2^(x - n) (fitted
+// as a linear program over 2001 Chebyshev points of [-0.5, 0.5]), times 2^n put together in the exponent field.
+// x is at most about 1 for an element that counts; -inf gives 0 exactly (n = -127: scale 0), NaN stays NaN.
+__device__ __forceinline__ float2 exp2_fma2(float2 x) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.x) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x.y) : "f"(-127.f));
+  const float2 t = __fadd2_rn(x, make_float2(kRoundMagic, kRoundMagic));
+  const float2 n = __fadd2_rn(t, make_float2(-kRoundMagic, -kRoundMagic));
+  const float2 r = __ffma2_rn(n, make_float2(-1.f, -1.f), x);
+  float2 q = __ffma2_rn(r, make_float2(0.001326472731307149f, 0.001326472731307149f),
+                        make_float2(0.009671512991189957f, 0.009671512991189957f));
+  q = __ffma2_rn(q, r, make_float2(0.05550733581185341f, 0.05550733581185341f));
+  q = __ffma2_rn(q, r, make_float2(0.24022242426872253f, 0.24022242426872253f));
+  q = __ffma2_rn(q, r, make_float2(0.6931470036506653f, 0.6931470036506653f));
+  q = __ffma2_rn(q, r, make_float2(1.f, 1.f));
+  return __fmul2_rn(q, make_float2(__int_as_float((__float_as_int(t.x) << 23) + 0x3F800000),
+                                   __int_as_float((__float_as_int(t.y) << 23) + 0x3F800000)));
+}
 
 // P = exp2(s * scale_log2 - M) for NS scores of a row (the whole row, or half of it in the two-pass
 // form), packed to 16-bit pairs; returns the sum of the unrounded exponentials. Packed two-wide fp32
