@@ -394,7 +394,7 @@ def run_ours(args, rank, local_rank, world):
     blk64_same = bool(torch.equal(out64, out))
     del out64
 
-    # ---- backward pass on the same workload (three launches per step), reported aside ---------------
+    # ---- backward pass on the same workload (two launches per step), reported aside ---------------
     bwd_ms = 0.0
     if not args.no_backward:
         from omni_attention_b200.ops import omni_attention_backward_out
@@ -490,9 +490,9 @@ def run_ours(args, rank, local_rank, world):
         # kernels execute seven (S and dP are recomputed by the dQ kernel)
         bwd_tf = 2.5 * flops / (bwd_ms * 1e-3) / 1e12
         line["backward"] = {"ms": bwd_ms, "value": 2.5 * flops_all / (bwd_ms * 1e-3) / 1e12, "unit": UNIT, "steps": 10,
-                            "launches_per_step": 3, "flop_count": "10*128*128*D per visited block",
+                            "launches_per_step": 2, "flop_count": "10*128*128*D per visited block",
                             "roofline_frac": bwd_tf / peak_tf,
-                            "kernels": "omni_bwd_prep_kernel, omni_bwd_dkdv_kernel, omni_bwd_dq_kernel"}
+                            "kernels": "omni_bwd_prep_kernel, omni_bwd_kernel"}
     if cap_ms > 0:
         line["softcap_forward"] = {"ms": cap_ms, "value": flops_all / (cap_ms * 1e-3) / 1e12, "unit": UNIT, "softcap": 50.0,
                                    "steps": 10, "roofline_frac": flops / (cap_ms * 1e-3) / 1e12 / peak_tf}

@@ -9,19 +9,20 @@
 //   dP = dO V^T,  delta = rowsum(dO * O),  dS = P * (dP - delta)
 //   dQ = scale * dS K,   dK = scale * dS^T Q
 //
-// Three launches on the caller's stream, all working memory in a caller-provided workspace:
+// Two launches on the caller's stream, all working memory in a caller-provided workspace:
 //   1. omni_bwd_prep_kernel   resolves every (Q block, KV block) of the lists into a dense table of
 //                             entry codes [BH, nq, nq] (so that the lists can be walked by column as
 //                             well as by row) and computes delta.
-//   2. omni_bwd_dkdv_kernel   one CTA per (KV block, batch*head): K, V stay in shared memory, the Q
-//                             blocks that visit this KV block stream through a two-stage ring; S^T and
+//   2. omni_bwd_kernel        two kinds of CTA:
+//      dK/dV                  one per (KV block, batch*head); K, V stay in shared memory, the Q
+//                             blocks that visit this KV block stream through a ring; S^T and
 //                             dP^T are computed transposed (TMEM lane = key) so that P^T and dS^T can be
 //                             fed to the tensor cores from TMEM for dV += P^T dO and dK += dS^T Q.
-//   3. omni_bwd_dq_kernel     one CTA per (Q block, batch*head), the mirror image: Q, dO stay, the
+//      dQ                     one per (Q block, batch*head), the mirror image: Q, dO stay, the
 //                             visited K, V stream; dQ += dS K with dS from TMEM.
-// S and dP are recomputed in both kernels (7 tile contractions per visited tile instead of 5), which
+// S and dP are recomputed in both kinds (7 tile contractions per visited tile instead of 5), which
 // buys a deterministic result with no atomics and no fp32 dQ buffer.
-// Both tile kernels are warp-specialised: 8 compute warps (a tile row = TMEM lane is shared by two
+// Both are warp-specialised: 8 compute warps (a tile row = TMEM lane is shared by two
 // threads, one per warpgroup, each taking 64 of its 128 columns), one warp whose first lane issues
 // every tcgen05.mma and one whose first lane issues the TMA loads; everything is handed over through
 // mbarriers (tcgen05.commit for "MMAs done", thread arrivals for "P / dS stored"). The per-element
@@ -47,7 +48,7 @@ struct BwdCfg {
   static constexpr int kVecBytes = 2 * kQStages * kBlock * 4;   // LSE and delta of a Q block
   static constexpr int kBitsBytes = 2 * kBlock * 16;      // bit-packed partial tiles of two visits
   static constexpr int kListBytes = kMaxKvBlocks * 4 + kMaxKvBlocks * 2 + 16;   // codes, visit list, its length
-  static constexpr int kSmemBytes = (4 + kQStages) * kTileBytes + kVecBytes + kBitsBytes + kListBytes + 256 + 1024;
+  static constexpr int kSmemBytes = (4 + kQStages) * kTileBytes + kVecBytes + kBitsBytes + kListBytes + 256;
 };
 
 // Of every eight element pairs, this many take their exponentials from the FMA pipe (exp2_fma2): the two halves of
@@ -76,7 +77,8 @@ __device__ __forceinline__ float2 unpack2(uint32_t w) {
 // 1. Workspace: entry-code table and delta. Grid (nq, BH), 160 threads: warps 0-3 compute delta of 32 rows
 // each, warp 4 resolves the Q block's list. Bound by the two 16-bit tensors read once, and for short batches by
 // load latency alone, so each warp has kBatch loads of 16 bytes per lane and tensor in flight, several rows at a
-// time (one row at a time, 4 bytes per lane: 25 us whatever the length below 2K tokens).
+// time (one row at a time, 4 bytes per lane: 24.7 against 4.7 us for 16 heads x 1.5K tokens, 34 against 27 for
+// 32 x 8K at D = 128, which is 5 TB/s).
 // ---------------------------------------------------------------------------------------------
 constexpr int kPrepThreads = 160;
 template <int D, bool BF16>
@@ -313,14 +315,9 @@ __device__ __forceinline__ float lse_to_log2(float lse) {
 // (32 heads x 4K tokens: 230 -> 211 us together with the vectors staged by the producer warp and kBwdPolyOf8.)
 // ---------------------------------------------------------------------------------------------
 template <int D, bool BF16, bool SOFTCAP>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                     const BwdParams p) {
+__device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                             const CUtensorMap& tmdO, const BwdParams& p, int cta, uint8_t* smem) {
   using Cfg = BwdCfg<D>;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  uint8_t* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
 
   const uint32_t sK = smem_u32(smem);
   const uint32_t sV = sK + Cfg::kTileBytes;
@@ -355,7 +352,7 @@ omni_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int t = tid & 127;          // key row of the tile = TMEM lane
   const int nq = p.f.nq;
   int kvb, bh;
-  bwd_decode_cta(p.f, static_cast<int>(blockIdx.x), false, kvb, bh);
+  bwd_decode_cta(p.f, cta, false, kvb, bh);
 
   if (tid == 0) {
     mbar_init(bar_kv, 1);
@@ -736,17 +733,9 @@ struct DqCfg {
 };
 
 template <int D, bool BF16, bool SOFTCAP>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                   const BwdParams p) {
+__device__ __forceinline__ void bwd_dq_cta(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                                           const CUtensorMap& tmdO, const BwdParams& p, int cta, uint8_t* smem) {
   using Cfg = DqCfg<D>;
-  extern __shared__ __align__(1024) uint8_t smem_dq[];
-  uint8_t* smem = smem_dq;
-  if ((smem_u32(smem) & 1023u) != 0u) {   // the swizzled tile layout needs it; uniform over the CTA
-    if (threadIdx.x == 0 && p.f.status != nullptr) atomicExch(p.f.status, kStatusWaitTimeout | (69 << 8));
-    return;
-  }
 
   const uint32_t sQ = smem_u32(smem);
   const uint32_t sdO = sQ + Cfg::kTileBytes;
@@ -773,7 +762,7 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int t = tid & 127;          // query row of the tile = TMEM lane
   const int nq = p.f.nq;
   int qb, bh;
-  bwd_decode_cta(p.f, static_cast<int>(blockIdx.x), true, qb, bh);
+  bwd_decode_cta(p.f, cta, true, qb, bh);
 
   if (tid == 0) {
     mbar_init(bar_qdo, 1);
@@ -978,27 +967,41 @@ omni_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
+// Both in one launch, the dK/dV CTAs first: neither needs the other's results, so the dQ CTAs fill the SMs that the
+// last dK/dV ones leave idle. That is most of a wave for short batches (16 heads x 12 blocks: 1.3 waves of each, 70.6 ->
+// 66.9 us with the soft-cap; 32 x 4K tokens at D = 64 369 -> 365, 32 x 8K at 128 1609 -> 1595; same bits).
+template <int D, bool BF16, bool SOFTCAP>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+omni_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                const __grid_constant__ BwdParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_bwd[];
+  if ((smem_u32(smem_bwd) & 1023u) != 0u) {   // the swizzled tile layout needs it; uniform over the CTA
+    if (threadIdx.x == 0 && p.f.status != nullptr) atomicExch(p.f.status, kStatusWaitTimeout | (69 << 8));
+    return;
+  }
+  const int ctas = p.f.nq * p.f.BH;
+  const int cta = static_cast<int>(blockIdx.x);
+  if (cta < ctas) {
+    bwd_dkdv_cta<D, BF16, SOFTCAP>(tmQ, tmK, tmV, tmdO, p, cta, smem_bwd);
+  } else {
+    bwd_dq_cta<D, BF16, SOFTCAP>(tmQ, tmK, tmV, tmdO, p, cta - ctas, smem_bwd);
+  }
+}
+
 template <int D, bool BF16, bool SOFTCAP>
 static cudaError_t launch_bwd_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                                 const CUtensorMap& tmdO, const BwdParams& p, cudaStream_t stream) {
-  using Cfg = BwdCfg<D>;
-  auto dkdv = omni_bwd_dkdv_kernel<D, BF16, SOFTCAP>;
-  auto dq = omni_bwd_dq_kernel<D, BF16, SOFTCAP>;
-  static SmemAttrOnce attr_dkdv[kMaxDevices];
-  static SmemAttrOnce attr_dq[kMaxDevices];
-  cudaError_t e = ensure_smem_attr(dkdv, Cfg::kSmemBytes, attr_dkdv);
+  constexpr int kSmem = BwdCfg<D>::kSmemBytes > DqCfg<D>::kSmemBytes ? BwdCfg<D>::kSmemBytes : DqCfg<D>::kSmemBytes;
+  auto kern = omni_bwd_kernel<D, BF16, SOFTCAP>;
+  static SmemAttrOnce attr[kMaxDevices];
+  cudaError_t e = ensure_smem_attr(kern, kSmem, attr);
   if (e != cudaSuccess) return e;
-  e = ensure_smem_attr(dq, DqCfg<D>::kSmemBytes, attr_dq);
-  if (e != cudaSuccess) return e;
-  const dim3 grid(p.f.nq, p.f.BH);
-  omni_bwd_prep_kernel<D, BF16><<<grid, kPrepThreads, 0, stream>>>(p);
+  omni_bwd_prep_kernel<D, BF16><<<dim3(p.f.nq, p.f.BH), kPrepThreads, 0, stream>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const unsigned ctas = static_cast<unsigned>(p.f.nq) * static_cast<unsigned>(p.f.BH);
-  dkdv<<<ctas, kBwdThreads, Cfg::kSmemBytes, stream>>>(tmQ, tmK, tmV, tmdO, p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  dq<<<ctas, kBwdThreads, DqCfg<D>::kSmemBytes, stream>>>(tmQ, tmK, tmV, tmdO, p);
+  kern<<<2 * ctas, kBwdThreads, kSmem, stream>>>(tmQ, tmK, tmV, tmdO, p);
   return cudaGetLastError();
 }
 

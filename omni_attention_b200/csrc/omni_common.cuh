@@ -238,17 +238,6 @@ __device__ __forceinline__ void load_partial_row(const FwdParams& p, uint32_t pi
   }
 }
 
-// One word of it (keys 32 * w .. 32 * w + 31).
-__device__ __forceinline__ uint32_t load_partial_word(const FwdParams& p, uint32_t pidx, int r, int w) {
-  const size_t row = static_cast<size_t>(pidx) * kBlock + r;
-  if (p.partial_bits != nullptr) return __ldg(p.partial_bits + row * 4 + w);
-  const uint4* src = reinterpret_cast<const uint4*>(p.partial_bool + row * kBlock) + 2 * w;
-  const uint4 a = __ldg(src), b = __ldg(src + 1);
-  return bytes_to_nibble(a.x) | (bytes_to_nibble(a.y) << 4) | (bytes_to_nibble(a.z) << 8) | (bytes_to_nibble(a.w) << 12) |
-         (bytes_to_nibble(b.x) << 16) | (bytes_to_nibble(b.y) << 20) | (bytes_to_nibble(b.z) << 24) |
-         (bytes_to_nibble(b.w) << 28);
-}
-
 // Allow-bits of row r for a diagonal CAUSAL tile: column c allowed iff c <= r.
 __device__ __forceinline__ void causal_row(int r, uint32_t (&allow)[4]) {
 #pragma unroll
