@@ -285,3 +285,18 @@ def test_small_and_odd_shapes_forward_and_backward(cuda_device, n, D):
     ref = orc.block_mask_attention_backward(pad(q), pad(k), pad(v), bm, pad(d_out), seqlen_orig=n)
     got = tuple(t.grad.float().cpu() for t in (qd, kd, vd))
     assert_grads(got, tuple(r[:, :, :n] for r in ref), torch.float16, all_heads(B, H), f"n={n} D={D}")
+
+
+@pytest.mark.parametrize("D,dtype", [(32, torch.float16), (64, torch.float16), (64, torch.bfloat16), (128, torch.bfloat16)])
+def test_every_number_of_visits(cuda_device, D, dtype):
+    """Nine blocks of random types below a CAUSAL diagonal, one column without a visitor: KV blocks visited by none to
+    nine Q blocks and the other way round, so that the rings of two and three stages wrap at every remainder."""
+    torch.manual_seed(17)
+    B, H, N = 1, 2, 9 * 128
+    bm = inputs.random_fcp_block_mask(B, H, N, seed=4)
+    bm.kv_num_blocks[:, :, 8] = 1   # the last Q block keeps one listed block; the last KV block has no visitor left
+    q, k, v, d_out = ((torch.randn(B, H, N, D) * 0.5).to(dtype) for _ in range(4))
+    ref = orc.block_mask_attention_backward(q, k, v, bm, d_out)
+    got = backward(q, k, v, d_out, bm, cuda_device)
+    assert_grads(got, ref, dtype, all_heads(B, H))
+    assert bool((got[1][:, :, -128:] == 0).all()) and bool((got[2][:, :, -128:] == 0).all())
