@@ -380,6 +380,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const float* x_other = xchg + (g ^ 1) * kXchgCols * kBlock + r;
         float2* ml = reinterpret_cast<float2*>(xchg + 2 * kXchgCols * kBlock);
         float f_mine = 0.f, f_other = 0.f;   // what the two accumulators are multiplied by
+        bool empty = true;                   // the row's output is zero whatever the accumulators hold (Inf, NaN)
 #pragma unroll
         for (int c = 0; c < D / 2 / kXchgCols; ++c, ++n_x) {
           const int col = g * (D / 2) + kXchgCols * c;   // finished here
@@ -409,7 +410,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             const float a_mine = st.M == -INFINITY ? 0.f : ex2_approx(st.M - M);
             const float a_other = o.x == -INFINITY ? 0.f : ex2_approx(o.x - M);
             const float l = st.l * a_mine + o.y * a_other;
-            const bool empty = q_abs >= p.seqlen_orig || M == -INFINITY || !(l > 0.f);
+            empty = q_abs >= p.seqlen_orig || M == -INFINITY || !(l > 0.f);
             const float inv = empty ? 0.f : 1.f / l;
             f_mine = a_mine * inv;
             f_other = a_other * inv;
@@ -422,7 +423,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int j = 0; j < kXchgCols / 2; ++j) {
             const float a = f_mine * __uint_as_float(own[2 * j]) + f_other * x_other[(2 * j) * kBlock];
             const float b = f_mine * __uint_as_float(own[2 * j + 1]) + f_other * x_other[(2 * j + 1) * kBlock];
-            w[j] = pack2<BF16>(a, b);
+            w[j] = pack2<BF16>(empty ? 0.f : a, empty ? 0.f : b);
           }
           mbar_arrive(bar_xfree + 8 * (g ^ 1));
           if (have_row && col < p.d_real) {

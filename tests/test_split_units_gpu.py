@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from conftest import assert_parity
-from omni_attention_b200 import omni_attention
+from omni_attention_b200 import create_causal_omni_block_mask, omni_attention, omni_attention_forward_out
 from omni_attention_b200.inputs import random_fcp_block_mask
 from oracle import omni_oracle as orc
 
@@ -37,3 +37,47 @@ def test_lists_of_any_length(cuda_device, H, nq, rest, D, dtype, block, softcap)
         assert_parity(got_o[live], got_l[live], ro[0, h][live], rl[0, h][live], f"head {h}")
     again = omni_attention(*(t.to(cuda_device) for t in (q, k, v)), bm, softcap=softcap)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("H", [2, 150])   # 150 heads of two tiles are more pairs than SMs: the pair form
+@pytest.mark.parametrize("D,dtype", [(32, torch.float16), (64, torch.bfloat16), (128, torch.bfloat16)])
+def test_rows_that_are_zero_whatever_the_inputs_hold(cuda_device, H, D, dtype):
+    """Rows beyond the sequence, rows without a key and rows with NaN scores are zero with log-sum-exp -inf in both
+    forms, also where q, k or v is not finite; every other row has the bits of the call on finite inputs."""
+    g = torch.Generator().manual_seed(D)
+    n, padded = 200, 256
+    q, k, v = (torch.randn(1, H, padded, D, generator=g).to(dtype).to(cuda_device) for _ in range(3))
+    bm = create_causal_omni_block_mask(1, H, n, n)
+    # the diagonal tile of the second Q block element by element, row 170 without any key there ...
+    tile = torch.ones(128, 128, dtype=torch.bool).tril()
+    tile[170 - 128] = False
+    bm.block_mask_types[:, :, 1, 1] = 3
+    bm.partial_block_mask_indices = torch.full_like(bm.kv_indices, -1)
+    bm.partial_block_mask_indices[:, :, 1, 1] = 0
+    bm.partial_block_masks = tile[None]
+    # ... and only that tile listed, so that row 170 attends nothing
+    bm.kv_num_blocks[:, :, 1] = 1
+    bm.kv_indices[:, :, 1, 0], bm.block_mask_types[:, :, 1, 0], bm.partial_block_mask_indices[:, :, 1, 0] = 1, 3, 0
+
+    def call(q, v):
+        out, lse = torch.full_like(q, 7.0), torch.zeros(1, H, padded, device=cuda_device)
+        omni_attention_forward_out(q, k, v, out, bm, n, lse=lse)
+        return out, lse
+
+    want, want_lse = call(q, v)
+    bad_q, bad_v = q.clone(), v.clone()
+    bad_q[:, :, n:] = float("nan")
+    bad_q[:, :, n + 3] = float("inf")
+    bad_q[:, :, 77, 3] = float("nan")
+    bad_v[:, :, 199, 5] = float("inf")   # key 199 is seen by row 199 alone, but its block is visited by all of the tile
+    out, lse = call(bad_q, bad_v)
+    zero = torch.zeros(padded, dtype=torch.bool, device=cuda_device)
+    zero[n:] = zero[77] = zero[170] = True
+    assert bool((out[:, :, zero] == 0).all()) and bool((lse[:, :, zero] == -float("inf")).all())
+    rest = ~zero
+    assert torch.equal(lse[:, :, rest], want_lse[:, :, rest])
+    first = rest.clone()
+    first[128:] = False
+    assert torch.equal(out[:, :, first], want[:, :, first])
+    cols = [c for c in range(D) if c != 5]   # 0 * Inf in column 5 of the rows that visit the block
+    assert torch.equal(out[:, :, rest][..., cols], want[:, :, rest][..., cols])
