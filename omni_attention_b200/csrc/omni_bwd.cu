@@ -336,12 +336,15 @@ __device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUten
   const uint32_t bar_do = smem_u32(bars + 4);       // [2] dO stage landed
   const uint32_t bar_s = smem_u32(bars + 6);        // [2] S^T of a visit complete (by visit parity)
   const uint32_t bar_dp = smem_u32(bars + 8);       // dP^T of the visit complete
-  const uint32_t bar_p = smem_u32(bars + 9);        // P^T stored (256 arrivals)
-  const uint32_t bar_ds = smem_u32(bars + 10);      // dS^T stored (256 arrivals)
-  const uint32_t bar_dvdone = smem_u32(bars + 11);  // [2] dV MMAs of the visit in this stage complete: dO stage free
-  const uint32_t bar_dkdone = smem_u32(bars + 13);  // [3] dK MMAs complete: Q, LSE and delta stage free
-  const uint32_t bar_vec = smem_u32(bars + 16);     // [3] LSE / delta of the visit in this stage written (32 arrivals)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  // [2] P^T of a visit stored (256 arrivals), by visit parity: with the scores issued a visit ahead, a warp can be
+  // through E1(i+1) while another is still in E1(i) and the issuer has not looked yet. Two are enough: E1(i+2)
+  // comes after E2(i+1), which needs dP^T(i+1), issued only after every thread has stored P^T(i) and dS^T(i).
+  const uint32_t bar_p = smem_u32(bars + 9);
+  const uint32_t bar_ds = smem_u32(bars + 11);      // dS^T stored (256 arrivals)
+  const uint32_t bar_dvdone = smem_u32(bars + 12);  // [2] dV MMAs of the visit in this stage complete: dO stage free
+  const uint32_t bar_dkdone = smem_u32(bars + 14);  // [3] dK MMAs complete: Q, LSE and delta stage free
+  const uint32_t bar_vec = smem_u32(bars + 17);     // [3] LSE / delta of the visit in this stage written (32 arrivals)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x;
@@ -365,9 +368,9 @@ __device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUten
       mbar_init(bar_do + 8 * s, 1);
       mbar_init(bar_dvdone + 8 * s, 1);
       mbar_init(bar_s + 8 * s, 1);
+      mbar_init(bar_p + 8 * s, kBwdComputeThreads);
     }
     mbar_init(bar_dp, 1);
-    mbar_init(bar_p, kBwdComputeThreads);
     mbar_init(bar_ds, kBwdComputeThreads);
     *abort_flag = 0;
     mbar_fence_init();
@@ -515,7 +518,7 @@ __device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUten
       const int stage = i & 1;
       const uint32_t ph = static_cast<uint32_t>(i & 1);
       // E1(i) has read S^T(i) and stored P^T(i) over it
-      mbar_wait(bar_p, ph, abort_flag, p.f.status, 58);
+      mbar_wait(bar_p + 8 * stage, static_cast<uint32_t>((i >> 1) & 1), abort_flag, p.f.status, 58);
       tc_fence_after();
       bwd_mma_ts_split<D>(tdV, region_s(i), 0, sdO + stage * Cfg::kTileBytes, idesc_ts, i > 0);    // dV += P^T(i) dO(i)
       tc_commit(bar_dvdone + 8 * stage);
@@ -649,7 +652,7 @@ __device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUten
       }
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(bar_p);
+      mbar_arrive(bar_p + 8 * (i & 1));
 
       if (i + 1 < n_vis) {
         next_qb = vis_s[i + 1];
