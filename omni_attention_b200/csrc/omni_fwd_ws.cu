@@ -856,6 +856,15 @@ static cudaError_t device_sm_count(int& sms) {
   return pd.err;
 }
 
+// Clearing the unit counter and the launch that draws from it belong together: two host threads on one stream that
+// share a counter could otherwise enqueue clear, clear, launch, launch, and the second kernel would find the units of
+// the first one taken. A lock for each of a few groups of counters, so that streams seldom wait for each other.
+static std::mutex& counter_lock(const void* counter) {
+  constexpr int kLocks = 16;   // scratch buffers are 256 bytes, from an allocator that aligns to as much
+  static std::mutex locks[kLocks];
+  return locks[(reinterpret_cast<uintptr_t>(counter) >> 8) % kLocks];
+}
+
 template <int D, bool BF16, bool SOFTCAP, bool B64, bool SPLIT>
 static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                                FwdParams p, cudaStream_t stream) {
@@ -896,7 +905,9 @@ static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
   // A grid that holds every unit hands out nothing (the kernel's first units are its block numbers and the
   // next of the fixed assignment does not exist), so the counter need not be cleared first.
   if (units <= grid) p.unit_counter = nullptr;
+  std::unique_lock<std::mutex> together;
   if (p.unit_counter != nullptr) {
+    together = std::unique_lock<std::mutex>(counter_lock(p.unit_counter));
     e = cudaMemsetAsync(p.unit_counter, 0, sizeof(int32_t), stream);
     if (e != cudaSuccess) return e;
   }

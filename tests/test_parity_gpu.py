@@ -456,6 +456,30 @@ def test_call_from_a_fresh_host_thread(cuda_device):
     assert torch.equal(out.cpu(), ref.cpu())
 
 
+def test_host_threads_on_one_stream(cuda_device):
+    """Four host threads that call the operator on the same stream at once, with more units than SMs: each call clears
+    the stream's unit counter and launches as one step, so none finds its units taken by another's."""
+    import threading
+
+    g = torch.Generator().manual_seed(8)
+    q, k, v = (torch.randn(1, 32, 1536, 64, generator=g).half().to(cuda_device) for _ in range(3))
+    bm = create_causal_omni_block_mask(1, 32, 1536, 1536)
+    want = omni_attention(q, k, v, bm)
+    wrong = []
+
+    def worker():
+        for _ in range(60):
+            outs = [omni_attention(q, k, v, bm) for _ in range(4)]
+            wrong.extend(not torch.equal(o, want) for o in outs)
+
+    threads = [threading.Thread(target=worker) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(wrong) == 4 * 60 * 4 and not any(wrong)
+
+
 def test_maximum_sequence_length(cuda_device):
     """1 024 KV blocks = 131 072 tokens, the most the kernels' per-CTA block tables hold: one head, causal
     lists with a FULL bidirectional band, sampled rows against the scalar oracle; the backward at the same
