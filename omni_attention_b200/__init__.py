@@ -27,23 +27,12 @@ __all__ = [
 
 
 def install_reference_module():
-    """Import the in-tree `omni_attn` pybind module and register it in sys.modules under that name
-    (the name omni-attn-mma/omni_attn_torch.py:539 imports)."""
-    import importlib.util
-    import os
+    """Register the in-tree `omni_attn` pybind module in sys.modules under that name (the name
+    omni-attn-mma/omni_attn_torch.py:539 imports) and return it. A module that is there already stays and is returned."""
     import sys
-    import sysconfig
 
-    import torch  # noqa: F401  (the extension links against libtorch)
+    from .ops import load_extension
 
-    if "omni_attn" in sys.modules:
-        return sys.modules["omni_attn"]
-    here = os.path.dirname(os.path.abspath(__file__))
-    path = os.path.join(here, "omni_attn" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
-    if not os.path.exists(path):
-        raise ImportError(f"{path} not found: build it with `python -m omni_attention_b200.build`")
-    spec = importlib.util.spec_from_file_location("omni_attn", path)
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    sys.modules["omni_attn"] = mod
-    return mod
+    if "omni_attn" not in sys.modules:
+        sys.modules["omni_attn"] = load_extension()
+    return sys.modules["omni_attn"]

@@ -17,8 +17,10 @@ device pointers. There is no CPU or PyTorch fallback: a missing library or a non
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import math
 import os
+import sysconfig
 from typing import Optional, Tuple, Union
 
 import torch
@@ -144,7 +146,7 @@ def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, s
     table (O(B*N*M) integer arithmetic). The kernels write the pool bit-packed, which is what the
     attention kernels read; the container's byte-per-element ``partial_block_masks`` is expanded from it
     only if somebody reads that field."""
-    res = _native().build_mask(modality_positions, batch, nheads, int(seq_len), int(padded),
+    res = load_extension().build_mask(modality_positions, batch, nheads, int(seq_len), int(padded),
                                device.index if device.index is not None else torch.cuda.current_device())
     if isinstance(res, int):
         _check(res)
@@ -205,13 +207,19 @@ def _device_mask(bm: OmniBlockMask, device: torch.device, pack_bits: bool) -> di
 _ext = None
 
 
-def _native():
-    """The in-tree extension module (built by ``omni_attention_b200.build``)."""
+def load_extension():
+    """The in-tree extension module (built by ``omni_attention_b200.build``). It is loaded by its path and kept here:
+    the operator neither reads nor sets ``sys.modules["omni_attn"]``, where a program may have the reference's own
+    extension (``install_reference_module`` registers this one there for those who ask)."""
     global _ext
     if _ext is None:
-        from . import install_reference_module
-
-        _ext = install_reference_module()
+        path = os.path.join(os.path.dirname(_LIB_PATH), "omni_attn" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python -m omni_attention_b200.build`")
+        spec = importlib.util.spec_from_file_location("omni_attn", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _ext = mod
     return _ext
 
 
@@ -221,7 +229,7 @@ def _native_mask(bm: OmniBlockMask, device: torch.device):
     if device.type != "cuda" or bm.Q_BLOCK_SIZE not in (64, 128) or bm.KV_BLOCK_SIZE != bm.Q_BLOCK_SIZE or bm.kv_len != bm.q_len:
         return None
     d = _device_mask(bm, device, True)
-    mask = _native().DeviceMask(d["nb"], d["idx"], d["typ"], d["pidx"], d["pbool"], d["pbits"], d["num_partial"],
+    mask = load_extension().DeviceMask(d["nb"], d["idx"], d["typ"], d["pidx"], d["pbool"], d["pbits"], d["num_partial"],
                                 bm.Q_BLOCK_SIZE, bm.q_len)
     bm._cache[device.index] = mask
     return mask
@@ -345,7 +353,7 @@ def omni_attention(query: Tensor, key: Tensor, value: Tensor, block_mask: OmniBl
             mask = _native_mask(block_mask, query.device)
         res = None
         if mask is not None:
-            res = _native().operator_forward(mask, query, key, value, scale or 0.0, _cap(softcap), return_lse)
+            res = load_extension().operator_forward(mask, query, key, value, scale or 0.0, _cap(softcap), return_lse)
         if res is None:
             _refuse(query, key, value, block_mask)
         if isinstance(res, int):
@@ -426,7 +434,7 @@ def omni_attention_autograd(query: Tensor, key: Tensor, value: Tensor, block_mas
         mask = _native_mask(block_mask, query.device)
     out = None
     if mask is not None:
-        out = _native().operator_autograd(mask, query, key, value, scale or 0.0, _cap(softcap))
+        out = load_extension().operator_autograd(mask, query, key, value, scale or 0.0, _cap(softcap))
     if out is None:
         _refuse(query, key, value, block_mask)
     return out

@@ -1,8 +1,11 @@
 """The C-ABI library loads without a GPU, exports every function include/omni_attn_sm100.h declares,
 and rejects bad arguments with the documented codes before touching the device."""
 import ctypes
+import json
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -44,6 +47,38 @@ def test_pybind_module_exports_reference_names():
     # the reference's wrappers pass 13 positional arguments; anything else is a TypeError
     with pytest.raises(TypeError):
         m.omni_attn_simple_kernel(1, 2, 3)
+
+
+def _python(code, **env):
+    """Runs ``code`` in a fresh interpreter; the last line of what it prints, as JSON."""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env={**os.environ, **env}, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return json.loads(r.stdout.strip().splitlines()[-1])
+
+
+def test_the_operator_does_not_use_or_take_the_module_name():
+    """The operator's extension is its own: another module called `omni_attn` in the process is neither used by it nor
+    replaced, and without one the name stays free until install_reference_module registers it."""
+    got = _python("""
+import json, sys, types
+import omni_attention_b200 as pkg
+from omni_attention_b200 import ops
+ext = ops.load_extension()
+free = "omni_attn" not in sys.modules
+mine = all(hasattr(ext, n) for n in ("DeviceMask", "operator_forward", "operator_autograd", "build_mask"))
+print(json.dumps([free, mine, pkg.install_reference_module() is ext, sys.modules["omni_attn"] is ext]))
+""")
+    assert got == [True, True, True, True]
+    got = _python("""
+import json, sys, types
+sys.modules["omni_attn"] = other = types.ModuleType("omni_attn")
+import omni_attention_b200 as pkg
+from omni_attention_b200 import ops
+ext = ops.load_extension()
+print(json.dumps([hasattr(ext, "DeviceMask"), sys.modules["omni_attn"] is other, pkg.install_reference_module() is other]))
+""")
+    assert got == [True, True, True]
 
 
 def _call(lib, fn="omni_attn_fwd_sm100", **kw):
