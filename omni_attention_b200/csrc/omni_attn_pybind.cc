@@ -11,6 +11,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <dlfcn.h>
 #include <torch/extension.h>
 
 #include <map>
@@ -26,6 +27,44 @@
 namespace {
 
 void fail(const std::string& msg) { throw std::runtime_error(msg); }
+
+// The C ABI this module calls: the library it is linked with, until use_library() names another build of it.
+struct Library {
+  decltype(&::omni_attn_fwd_simple_sm100) fwd_simple = &::omni_attn_fwd_simple_sm100;
+  decltype(&::omni_attn_fwd_scratch_sm100) fwd_scratch = &::omni_attn_fwd_scratch_sm100;
+  decltype(&::omni_attn_fwd_rows_sm100) fwd_rows = &::omni_attn_fwd_rows_sm100;
+  decltype(&::omni_attn_bwd_ex_sm100) bwd_ex = &::omni_attn_bwd_ex_sm100;
+  decltype(&::omni_attn_bwd_rows_sm100) bwd_rows = &::omni_attn_bwd_rows_sm100;
+  decltype(&::omni_attn_build_mask_sm100) build_mask = &::omni_attn_build_mask_sm100;
+  decltype(&::omni_attn_bwd_workspace_bytes) bwd_workspace_bytes = &::omni_attn_bwd_workspace_bytes;
+  decltype(&::omni_attn_error_string) error_string = &::omni_attn_error_string;
+  decltype(&::omni_attn_last_cuda_error) last_cuda_error = &::omni_attn_last_cuda_error;
+};
+Library library;
+
+template <typename Fn>
+void look_up(void* handle, const char* name, Fn& fn) {
+  void* at = dlsym(handle, name);
+  if (at == nullptr) fail(std::string("no function ") + name + " in the library given");
+  fn = reinterpret_cast<Fn>(at);
+}
+
+// Called once, before the module is used.
+void use_library(const std::string& path) {
+  void* handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (handle == nullptr) fail(dlerror());
+  Library found;
+  look_up(handle, "omni_attn_fwd_simple_sm100", found.fwd_simple);
+  look_up(handle, "omni_attn_fwd_scratch_sm100", found.fwd_scratch);
+  look_up(handle, "omni_attn_fwd_rows_sm100", found.fwd_rows);
+  look_up(handle, "omni_attn_bwd_ex_sm100", found.bwd_ex);
+  look_up(handle, "omni_attn_bwd_rows_sm100", found.bwd_rows);
+  look_up(handle, "omni_attn_build_mask_sm100", found.build_mask);
+  look_up(handle, "omni_attn_bwd_workspace_bytes", found.bwd_workspace_bytes);
+  look_up(handle, "omni_attn_error_string", found.error_string);
+  look_up(handle, "omni_attn_last_cuda_error", found.last_cuda_error);
+  library = found;
+}
 
 void check_qkvo(const torch::Tensor& t, const char* name, c10::ScalarType dtype) {
   if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor");
@@ -159,22 +198,22 @@ void forward_impl(bool simple, const torch::Tensor& Q, const torch::Tensor& K, c
   const int dt = dtype == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16;
   int rc;
   if (simple) {
-    rc = omni_attn_fwd_simple_sm100(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse_ptr,
-                                    kv_num_blocks.data_ptr<int32_t>(), kv_indices.data_ptr<int32_t>(),
-                                    block_mask_types.data_ptr<int32_t>(), pidx, pbool, pbits, B, H, N, seqlen_orig, D,
-                                    Q_BLOCK_SIZE, KV_BLOCK_SIZE, max_blocks, num_partial, dt, static_cast<float>(scale),
-                                    stream, status_ptr);
+    rc = library.fwd_simple(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse_ptr,
+                            kv_num_blocks.data_ptr<int32_t>(), kv_indices.data_ptr<int32_t>(),
+                            block_mask_types.data_ptr<int32_t>(), pidx, pbool, pbits, B, H, N, seqlen_orig, D,
+                            Q_BLOCK_SIZE, KV_BLOCK_SIZE, max_blocks, num_partial, dt, static_cast<float>(scale),
+                            stream, status_ptr);
   } else {
-    rc = omni_attn_fwd_scratch_sm100(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse_ptr,
-                                     kv_num_blocks.data_ptr<int32_t>(), kv_indices.data_ptr<int32_t>(),
-                                     block_mask_types.data_ptr<int32_t>(), pidx, pbool, pbits, B, H, N, seqlen_orig, D,
-                                     Q_BLOCK_SIZE, KV_BLOCK_SIZE, max_blocks, num_partial, dt, static_cast<float>(scale),
-                                     stream, status_ptr, stream_scratch(Q, stream), OMNI_ATTN_SCRATCH_BYTES);
+    rc = library.fwd_scratch(Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse_ptr,
+                             kv_num_blocks.data_ptr<int32_t>(), kv_indices.data_ptr<int32_t>(),
+                             block_mask_types.data_ptr<int32_t>(), pidx, pbool, pbits, B, H, N, seqlen_orig, D,
+                             Q_BLOCK_SIZE, KV_BLOCK_SIZE, max_blocks, num_partial, dt, static_cast<float>(scale),
+                             stream, status_ptr, stream_scratch(Q, stream), OMNI_ATTN_SCRATCH_BYTES);
   }
   if (rc != OMNI_OK) {
     std::ostringstream os;
-    os << "omni_attn forward failed: " << omni_attn_error_string(rc) << " (code " << rc;
-    if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << omni_attn_last_cuda_error();
+    os << "omni_attn forward failed: " << library.error_string(rc) << " (code " << rc;
+    if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << library.last_cuda_error();
     os << ")";
     fail(os.str());
   }
@@ -279,7 +318,7 @@ void omni_attn_bwd(torch::Tensor Q, torch::Tensor K, torch::Tensor V, torch::Ten
   }
   c10::cuda::CUDAGuard guard(Q.device());
   cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-  const int rc = omni_attn_bwd_ex_sm100(
+  const int rc = library.bwd_ex(
       Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), lse.data_ptr<float>(), dO.data_ptr(), dQ.data_ptr(),
       dK.data_ptr(), dV.data_ptr(), kv_num_blocks.data_ptr<int32_t>(), kv_indices.data_ptr<int32_t>(),
       block_mask_types.data_ptr<int32_t>(), pidx, pbool, pbits, B, H, N, seqlen_orig, D, Q_BLOCK_SIZE, KV_BLOCK_SIZE,
@@ -289,15 +328,15 @@ void omni_attn_bwd(torch::Tensor Q, torch::Tensor K, torch::Tensor V, torch::Ten
       static_cast<float>(softcap));
   if (rc != OMNI_OK) {
     std::ostringstream os;
-    os << "omni_attn backward failed: " << omni_attn_error_string(rc) << " (code " << rc;
-    if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << omni_attn_last_cuda_error();
+    os << "omni_attn backward failed: " << library.error_string(rc) << " (code " << rc;
+    if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << library.last_cuda_error();
     os << ")";
     fail(os.str());
   }
 }
 
 long long omni_attn_bwd_workspace(int B, int H, int seqlen_padded) {
-  return omni_attn_bwd_workspace_bytes(B, H, seqlen_padded);
+  return library.bwd_workspace_bytes(B, H, seqlen_padded);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -379,13 +418,13 @@ int forward_call(DeviceMask& m, const torch::Tensor& q, const torch::Tensor& k, 
   const auto stream = at::cuda::getCurrentCUDAStream();
   m.order_after_build(stream);
   const int n = static_cast<int>(q.size(2));
-  return omni_attn_fwd_rows_sm100(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse,
-                                  m.nb.data_ptr<int32_t>(), m.idx.data_ptr<int32_t>(), m.types.data_ptr<int32_t>(),
-                                  m.partial_idx_ptr(), m.partial_bool_ptr(), m.partial_bits_ptr(), m.B, m.H, m.padded, n,
-                                  static_cast<int>(q.size(3)), m.block, m.block, m.max_blocks, m.num_partial,
-                                  q.scalar_type() == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16,
-                                  static_cast<float>(scale), stream.stream(), nullptr, n, static_cast<float>(softcap),
-                                  stream_scratch(q, stream.stream()), OMNI_ATTN_SCRATCH_BYTES);
+  return library.fwd_rows(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse,
+                          m.nb.data_ptr<int32_t>(), m.idx.data_ptr<int32_t>(), m.types.data_ptr<int32_t>(),
+                          m.partial_idx_ptr(), m.partial_bool_ptr(), m.partial_bits_ptr(), m.B, m.H, m.padded, n,
+                          static_cast<int>(q.size(3)), m.block, m.block, m.max_blocks, m.num_partial,
+                          q.scalar_type() == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16,
+                          static_cast<float>(scale), stream.stream(), nullptr, n, static_cast<float>(softcap),
+                          stream_scratch(q, stream.stream()), OMNI_ATTN_SCRATCH_BYTES);
 }
 
 // Contiguous, and for a length that is no multiple of the block (callers of such lengths may pass any view)
@@ -420,8 +459,8 @@ pybind11::object operator_forward(const MaskPtr& m, torch::Tensor q, torch::Tens
 
 void throw_rc(const char* what, int rc) {
   std::ostringstream os;
-  os << what << ": " << omni_attn_error_string(rc) << " (code " << rc;
-  if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << omni_attn_last_cuda_error();
+  os << what << ": " << library.error_string(rc) << " (code " << rc;
+  if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << library.last_cuda_error();
   os << ")";
   fail(os.str());
 }
@@ -449,12 +488,12 @@ struct OmniAttentionFn : torch::autograd::Function<OmniAttentionFn> {
     const auto d_out = packed(grads[0], *mask);
     auto dq = at::empty(q.sizes(), q.options()), dk = at::empty(q.sizes(), q.options()),
          dv = at::empty(q.sizes(), q.options());
-    const long long need = omni_attn_bwd_workspace_bytes(mask->B, mask->H, mask->padded);
+    const long long need = library.bwd_workspace_bytes(mask->B, mask->H, mask->padded);
     auto workspace = at::empty({need}, q.options().dtype(torch::kUInt8));
     const auto stream = at::cuda::getCurrentCUDAStream();
     mask->order_after_build(stream);
     const int n = static_cast<int>(q.size(2));
-    const int rc = omni_attn_bwd_rows_sm100(
+    const int rc = library.bwd_rows(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), d_out.data_ptr(),
         dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), mask->nb.data_ptr<int32_t>(), mask->idx.data_ptr<int32_t>(),
         mask->types.data_ptr<int32_t>(), mask->partial_idx_ptr(), mask->partial_bool_ptr(), mask->partial_bits_ptr(),
@@ -503,12 +542,12 @@ pybind11::object build_mask(torch::Tensor modality_positions, int B, int H, int 
     bits = at::empty({capacity, 128, 4}, opt);
     count = at::empty({1}, opt);
     scratch = at::empty({2 * B * nq}, opt);
-    rc = omni_attn_build_mask_sm100(mp.numel() > 0 ? mp.data_ptr<int32_t>() : nullptr, B, static_cast<int>(mp.size(1)), H,
-                                    seqlen, padded, nb.data_ptr<int32_t>(), idx.data_ptr<int32_t>(),
-                                    types.data_ptr<int32_t>(), pidx.data_ptr<int32_t>(),
-                                    reinterpret_cast<uint32_t*>(bits.data_ptr<int32_t>()), nullptr, capacity,
-                                    count.data_ptr<int32_t>(), scratch.data_ptr<int32_t>(),
-                                    static_cast<long long>(scratch.numel()) * 4, at::cuda::getCurrentCUDAStream().stream());
+    rc = library.build_mask(mp.numel() > 0 ? mp.data_ptr<int32_t>() : nullptr, B, static_cast<int>(mp.size(1)), H,
+                            seqlen, padded, nb.data_ptr<int32_t>(), idx.data_ptr<int32_t>(),
+                            types.data_ptr<int32_t>(), pidx.data_ptr<int32_t>(),
+                            reinterpret_cast<uint32_t*>(bits.data_ptr<int32_t>()), nullptr, capacity,
+                            count.data_ptr<int32_t>(), scratch.data_ptr<int32_t>(),
+                            static_cast<long long>(scratch.numel()) * 4, at::cuda::getCurrentCUDAStream().stream());
     if (rc == OMNI_OK) {
       mask = c10::make_intrusive<DeviceMask>(nb, idx, types, pidx, std::nullopt, bits, capacity, 128, padded);
     }
@@ -545,6 +584,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("has_partial"), pybind11::arg("workspace"), pybind11::arg("scale") = pybind11::none(),
         pybind11::arg("status") = pybind11::none(), pybind11::arg("partial_bits") = pybind11::none(),
         pybind11::arg("softcap") = 0.0);
+  m.def("use_library", &use_library, "calls another build of libomni_attn_sm100.so from here on");
   pybind11::class_<DeviceMask, MaskPtr>(m, "DeviceMask", "device-side form of a block mask")
       .def(pybind11::init([](torch::Tensor nb, torch::Tensor idx, torch::Tensor types, std::optional<torch::Tensor> pidx,
                              std::optional<torch::Tensor> pbool, std::optional<torch::Tensor> pbits, int num_partial,

@@ -64,7 +64,8 @@ class OmniAttnError(RuntimeError):
 
 def load_library() -> ctypes.CDLL:
     """Load libomni_attn_sm100.so from the package directory (built by ``omni_attention_b200.build``);
-    the environment variable OMNI_ATTN_LIBRARY names another build of the same library."""
+    the environment variable OMNI_ATTN_LIBRARY names another build of the same library, which the extension module
+    then calls too."""
     global _lib
     if _lib is not None:
         return _lib
@@ -219,6 +220,9 @@ def load_extension():
         spec = importlib.util.spec_from_file_location("omni_attn", path)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
+        lib = load_library()._name
+        if os.path.realpath(lib) != os.path.realpath(_LIB_PATH):   # OMNI_ATTN_LIBRARY
+            mod.use_library(os.path.abspath(lib))
         _ext = mod
     return _ext
 

@@ -81,6 +81,29 @@ print(json.dumps([hasattr(ext, "DeviceMask"), sys.modules["omni_attn"] is other,
     assert got == [True, True, True]
 
 
+def test_the_library_named_by_the_environment_is_the_one_the_operator_calls(tmp_path):
+    """A stand-in with every function of the ABI, whose workspace size is its own: both ways into the library, ctypes and
+    the extension module (also as the reference's module), must end there. Without a function it is refused."""
+    build = lambda name, body: subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / name), "-x", "c", "-"],
+                                              input=body, text=True, check=True)
+    code = """
+import json
+import omni_attention_b200 as pkg
+from omni_attention_b200 import ops
+a = ops.load_library().omni_attn_bwd_workspace_bytes(1, 1, 128)
+print(json.dumps([a, ops.load_extension().omni_attn_bwd_workspace_bytes(1, 1, 128),
+                  pkg.install_reference_module().omni_attn_bwd_workspace_bytes(1, 1, 128)]))
+"""
+    body = "".join(f"long long {n}(void) {{ return 4711; }}\n" for n in ops.ABI_SYMBOLS)
+    build("other.so", body)
+    assert _python(code, OMNI_ATTN_LIBRARY=str(tmp_path / "other.so")) == [4711] * 3
+    own = ops.load_library().omni_attn_bwd_workspace_bytes(1, 1, 128)
+    assert own != 4711 and _python(code) == [own] * 3
+    build("short.so", body.replace("omni_attn_bwd_rows_sm100", "something_else"))
+    with pytest.raises(AssertionError, match="omni_attn_bwd_rows_sm100"):
+        _python(code, OMNI_ATTN_LIBRARY=str(tmp_path / "short.so"))
+
+
 def _call(lib, fn="omni_attn_fwd_sm100", **kw):
     buf = (ctypes.c_char * 4096)()
     a = ctypes.addressof(buf)
