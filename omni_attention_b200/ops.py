@@ -430,7 +430,6 @@ def omni_attention_autograd(query: Tensor, key: Tensor, value: Tensor, block_mas
         # the backward kernels take 128-blocks: re-expressed quadrant by quadrant, once per mask object
         hit = block_mask._cache.get("retiled128")
         if hit is None:
-            _check_shapes(query, key, value, block_mask)
             hit = block_mask._cache["retiled128"] = retile_block_mask(block_mask, 128)
         block_mask = hit
     mask = block_mask._cache.get(query.get_device())

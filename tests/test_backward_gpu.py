@@ -326,3 +326,25 @@ def test_warps_that_take_unequally_long(cuda_device, D, dtype):
         assert all(torch.equal(a, b) for a, b in zip(got, first))
     ref = orc.block_mask_attention_backward(q, k, v, bm, d_out, softcap=cap)
     assert_grads(tuple(t.float().cpu() for t in first), ref, dtype, all_heads(B, H))
+
+
+@pytest.mark.parametrize("used_before", [False, True])
+def test_any_length_that_the_retiled_mask_holds(cuda_device, used_before):
+    """Training on a 64-block mask runs on the mask's 128-tiles, so every length that pads to those is taken, also one
+    beyond the 64-block mask's own length (its rows there attend nothing), whether the mask was used before or not; a length
+    that does not is refused."""
+    g = torch.Generator().manual_seed(3)
+    bm = create_causal_omni_block_mask(1, 2, 320, 320, 64, 64)
+    make = lambda n: [torch.randn(1, 2, n, 64, generator=g).half().to(cuda_device).requires_grad_(True) for _ in range(3)]
+    if used_before:
+        omni_attention_autograd(*make(300), bm)
+    q, k, v = make(350)
+    out = omni_attention_autograd(q, k, v, bm)
+    grads = torch.autograd.grad(out, (q, k, v), torch.ones_like(out))
+    assert all(bool((t[:, :, 320:] == 0).all()) for t in (out, *grads))
+    head = [t.detach()[:, :, :320].contiguous() for t in (q, k, v)]
+    assert torch.equal(out[:, :, :320], omni_attention_autograd(*head, bm))
+    with pytest.raises(ops.OmniAttnError, match="padded length"):
+        omni_attention_autograd(*make(256), bm)
+    with pytest.raises(ValueError, match="head_dim"):
+        omni_attention_autograd(*(torch.zeros(1, 2, 320, 96, dtype=torch.float16, device=cuda_device),) * 3, bm)
