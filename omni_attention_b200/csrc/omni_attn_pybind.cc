@@ -346,6 +346,26 @@ long long omni_attn_bwd_workspace(int B, int H, int seqlen_padded) {
 // of a forward + backward about 80 us; the kernels of a 512-token call take 15.)
 // -------------------------------------------------------------------------------------------------
 
+// The Python package's exception class, which every refusal of the operator is; any thread may raise it, an
+// autograd worker too.
+PyObject* operator_error = PyExc_RuntimeError;
+
+void set_error_type(pybind11::object type) { operator_error = type.release().ptr(); }
+
+[[noreturn]] void refuse(const std::string& msg) {
+  pybind11::gil_scoped_acquire gil;
+  PyErr_SetString(operator_error, msg.c_str());
+  throw pybind11::error_already_set();
+}
+
+[[noreturn]] void refuse(int rc) {
+  std::ostringstream os;
+  os << "omni_attn: " << library.error_string(rc) << " (code " << rc;
+  if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << library.last_cuda_error();
+  os << ")";
+  refuse(os.str());
+}
+
 // Device-side form of one OmniBlockMask: int32 lists, bit-packed (or byte) pool. Built once per mask object
 // and device by the Python side, which keeps it on the mask. The copies were enqueued on the stream that
 // was current at construction; a call on another stream waits for them.
@@ -366,12 +386,12 @@ struct DeviceMask : torch::CustomClassHolder {
     check_index(types, "block_mask_types");
     if (nb.dim() != 3 || idx.dim() != 4 || idx.size(0) != nb.size(0) || idx.size(1) != nb.size(1) ||
         idx.size(2) != nb.size(2) || types.sizes() != idx.sizes()) {
-      fail("kv_num_blocks must be [B, H, nq]; kv_indices and block_mask_types [B, H, nq, max_blocks]");
+      refuse("kv_num_blocks must be [B, H, nq]; kv_indices and block_mask_types [B, H, nq, max_blocks]: shape mismatch");
     }
     if (pidx_.has_value()) {
       pidx = *pidx_;
       check_index(pidx, "partial_block_mask_indices");
-      if (pidx.sizes() != idx.sizes()) fail("partial_block_mask_indices must have the shape of kv_indices");
+      if (pidx.sizes() != idx.sizes()) refuse("partial_block_mask_indices must have the shape of kv_indices: shape mismatch");
     }
     if (pbool_.has_value()) pbool = *pbool_;
     if (pbits_.has_value()) pbits = *pbits_;
@@ -457,21 +477,13 @@ pybind11::object operator_forward(const MaskPtr& m, torch::Tensor q, torch::Tens
   return pybind11::cast(out);
 }
 
-void throw_rc(const char* what, int rc) {
-  std::ostringstream os;
-  os << what << ": " << library.error_string(rc) << " (code " << rc;
-  if (rc == OMNI_ERR_CUDA) os << ", CUDA error " << library.last_cuda_error();
-  os << ")";
-  fail(os.str());
-}
-
 struct OmniAttentionFn : torch::autograd::Function<OmniAttentionFn> {
   static torch::Tensor forward(torch::autograd::AutogradContext* ctx, const torch::Tensor& q, const torch::Tensor& k,
                                const torch::Tensor& v, const MaskPtr& mask, double scale, double softcap) {
     auto out = at::empty(q.sizes(), q.options());
     auto lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(torch::kFloat32));
     const int rc = forward_call(*mask, q, k, v, out, lse.data_ptr<float>(), scale, softcap);
-    if (rc != OMNI_OK) throw_rc("omni_attn", rc);
+    if (rc != OMNI_OK) refuse(rc);
     ctx->save_for_backward({q, k, v, out, lse});
     ctx->saved_data["mask"] = c10::IValue::make_capsule(mask);
     ctx->saved_data["scale"] = scale;
@@ -501,7 +513,7 @@ struct OmniAttentionFn : torch::autograd::Function<OmniAttentionFn> {
         mask->num_partial, q.scalar_type() == torch::kBFloat16 ? OMNI_DTYPE_BF16 : OMNI_DTYPE_F16,
         static_cast<float>(ctx->saved_data["scale"].toDouble()), stream.stream(), nullptr, workspace.data_ptr(), need,
         static_cast<float>(ctx->saved_data["softcap"].toDouble()), n);
-    if (rc != OMNI_OK) throw_rc("omni_attn", rc);
+    if (rc != OMNI_OK) refuse(rc);
     return {dq, dk, dv, torch::Tensor(), torch::Tensor(), torch::Tensor()};
   }
 };
@@ -585,6 +597,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("status") = pybind11::none(), pybind11::arg("partial_bits") = pybind11::none(),
         pybind11::arg("softcap") = 0.0);
   m.def("use_library", &use_library, "calls another build of libomni_attn_sm100.so from here on");
+  m.def("set_error_type", &set_error_type, "the class of what the operator raises");
   pybind11::class_<DeviceMask, MaskPtr>(m, "DeviceMask", "device-side form of a block mask")
       .def(pybind11::init([](torch::Tensor nb, torch::Tensor idx, torch::Tensor types, std::optional<torch::Tensor> pidx,
                              std::optional<torch::Tensor> pbool, std::optional<torch::Tensor> pbits, int num_partial,

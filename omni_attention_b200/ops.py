@@ -223,6 +223,7 @@ def load_extension():
         lib = load_library()._name
         if os.path.realpath(lib) != os.path.realpath(_LIB_PATH):   # OMNI_ATTN_LIBRARY
             mod.use_library(os.path.abspath(lib))
+        mod.set_error_type(OmniAttnError)
         _ext = mod
     return _ext
 

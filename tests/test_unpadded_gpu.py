@@ -5,7 +5,7 @@ import torch
 
 from omni_attention_b200 import (block_mask_from_row_limits, create_omni_block_mask_from_modality_positions as build_mask,
                                  omni_attention, omni_attention_autograd, retile_block_mask)
-from omni_attention_b200.ops import omni_attention_backward_out, omni_attention_forward_out
+from omni_attention_b200.ops import OmniAttnError, omni_attention_backward_out, omni_attention_forward_out
 
 pytestmark = pytest.mark.gpu
 
@@ -91,6 +91,29 @@ def test_views_that_start_at_any_element(cuda_device, n):
 
     for a, b in zip(grads((q, k, v), do), grads([t.clone() for t in (q, k, v)], do.clone())):
         assert torch.equal(a, b)
+
+
+def test_every_refusal_is_an_omni_attn_error(cuda_device):
+    """Unaligned tensors of whole blocks, forward and backward, and lists whose shapes do not fit each other or q."""
+    n, numel = 256, 2 * 256 * 64
+    flat = torch.randn(numel + 8, device=cuda_device).half()
+    unaligned, q = flat[1:1 + numel].view(1, 2, n, 64), flat[:numel].view(1, 2, n, 64)
+    mask = lambda: block_mask_from_row_limits(torch.arange(n).view(1, n), 2)
+    bm = mask()
+    for call in (omni_attention, omni_attention_autograd):
+        with pytest.raises(OmniAttnError, match="aligned"):
+            call(unaligned, unaligned, unaligned, bm)
+    leaf = q.clone().requires_grad_(True)
+    out = omni_attention_autograd(leaf, leaf, leaf, bm)
+    with pytest.raises(OmniAttnError, match="aligned"):
+        out.backward(unaligned)
+    for name, cut in (("block_mask_types", lambda t: t[..., :1]), ("kv_num_blocks", lambda t: t[:, :1]),
+                      ("kv_indices", lambda t: t[:, :1])):
+        for call in (omni_attention, omni_attention_autograd):
+            bad = mask()
+            setattr(bad, name, cut(getattr(bad, name)))
+            with pytest.raises(OmniAttnError):
+                call(q, q, q, bad)
 
 
 @pytest.mark.parametrize("softcap", [0.0, -1.0, float("nan")])
