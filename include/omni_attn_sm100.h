@@ -249,7 +249,7 @@ void omni_attn_set_wait_cycles(long long cycles);
  *  num_partial_out     out, one device int32: PARTIAL tiles the mask needs; when it exceeds
  *                      partial_capacity the tiles beyond the capacity were not written and the call must
  *                      be repeated with a larger pool
- *  scratch             device memory, at least 2 * B * nq * 4 bytes
+ *  scratch             device memory, at least 2 * B * nq * 4 bytes (used by batches of many Q blocks)
  * Block types by content: all elements allowed -> FULL, none -> not listed, a diagonal block of plain
  * causal rows -> CAUSAL, anything else -> PARTIAL (the derivation of
  * omni-attn-mma/generate_attn_data.py:200-236; the reference builder's "dominant type" shortcut types

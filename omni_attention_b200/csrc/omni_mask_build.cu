@@ -19,11 +19,13 @@
 //
 // limit(q) never decreases inside the sequence, so the limits of a block are those of its first and last
 // row, the listed KV blocks are 0 .. limit_max / 128, the first (limit_min + 1) / 128 of them FULL, and
-// everything there is to know about a Q block takes one pass over the spans. One kernel therefore does
-// it all: a CTA works out its own Q block and, for the position of its PARTIAL tiles in the pool, the
+// everything there is to know about a Q block takes one pass over the spans. For few blocks one kernel therefore
+// does it all: a CTA works out its own Q block and, for the position of its PARTIAL tiles in the pool, the
 // PARTIAL counts of all Q blocks before it (the counts of a thread's share of them, summed over the CTA),
-// writes its pool tiles and the lists of a slice of the heads. HBM-write bound for long sequences (the index
-// tensors: 101 MB for a 4 x 32-head batch of 32K tokens), one launch latency for short ones.
+// writes its pool tiles and the lists of a slice of the heads. That counting grows with the square of the number of
+// Q blocks in the batch; where it would take longer than two small launches (see count_first) the blocks are
+// counted once and the counts summed up in the caller's scratch first. HBM-write bound for long sequences (the index
+// tensors: 101 MB for a 4 x 32-head batch of 32K tokens), launch latency for short ones.
 #include <cstdint>
 
 #include "../../include/omni_attn_sm100.h"
@@ -43,6 +45,8 @@ struct MaskParams {
   uint32_t* partial_bits;             // [capacity, 128, 4]
   uint8_t* partial_bool;              // [capacity, 128, 128] or null
   int32_t* num_partial_out;           // device int
+  int32_t* counts;                    // [B, nq] PARTIAL tiles of each Q block, and
+  int32_t* bases;                     // [B, nq] of all before it; null when every CTA counts for itself
   int B, M, H, seqlen, nq, capacity;
   int heads_per_cta;                  // heads whose lists one CTA writes (grid z = slices of the heads)
   bool vec4;                          // list rows are 16-byte aligned
@@ -93,20 +97,55 @@ __device__ __forceinline__ BlockShape block_shape(const MaskParams& p, int b, in
   return s;
 }
 
+__global__ void __launch_bounds__(kMaskThreads) mask_count_kernel(const MaskParams p) {
+  const int i = blockIdx.x * kMaskThreads + threadIdx.x;
+  if (i < p.B * p.nq) p.counts[i] = block_shape(p, i / p.nq, i % p.nq).partials(i % p.nq);
+}
+
+// Exclusive prefix sums of the counts, one CTA: each thread sums a run of neighbours, then writes their bases.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads) mask_scan_kernel(const MaskParams p) {
+  __shared__ int warp_sum[kScanThreads / 32];
+  const int t = threadIdx.x, n = p.B * p.nq;
+  const int run = (n + kScanThreads - 1) / kScanThreads;
+  const int first = min(n, t * run), last = min(n, first + run);
+  int sum = 0;
+  for (int i = first; i < last; ++i) sum += p.counts[i];
+  int upto = sum;   // of the threads up to this one
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+    if ((t & 31) >= o) upto += x;
+  }
+  if ((t & 31) == 31) warp_sum[t >> 5] = upto;
+  __syncthreads();
+  int base = upto - sum;
+  for (int w = 0; w < (t >> 5); ++w) base += warp_sum[w];
+  for (int i = first; i < last; ++i) {
+    p.bases[i] = base;
+    base += p.counts[i];
+  }
+}
+
 __global__ void __launch_bounds__(kMaskThreads) mask_build_kernel(const MaskParams p) {
   __shared__ int part[kMaskThreads / 32];
   const int qb = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
   const BlockShape own = block_shape(p, b, qb);
 
   // pool position of this block's first PARTIAL tile
-  int before = 0;
   const int me = b * p.nq + qb;
-  for (int i = t; i < me; i += kMaskThreads) before += block_shape(p, i / p.nq, i % p.nq).partials(i % p.nq);
+  int base;
+  if (p.bases != nullptr) {
+    base = p.bases[me];
+  } else {
+    int before = 0;
+    for (int i = t; i < me; i += kMaskThreads) before += block_shape(p, i / p.nq, i % p.nq).partials(i % p.nq);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
-  if ((t & 31) == 0) part[t >> 5] = before;
-  __syncthreads();
-  const int base = part[0] + part[1] + part[2] + part[3];
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
+    if ((t & 31) == 0) part[t >> 5] = before;
+    __syncthreads();
+    base = part[0] + part[1] + part[2] + part[3];
+  }
   const bool diag = own.diag_in_range(qb);
 
   if (blockIdx.z == 0) {   // the pool, shared by the heads: thread t writes row t of every PARTIAL tile
@@ -182,6 +221,16 @@ __global__ void __launch_bounds__(kMaskThreads) mask_build_kernel(const MaskPara
   for (int h = h0 + t; h < h1; h += kMaskThreads) p.kv_num_blocks[(static_cast<long long>(b) * p.H + h) * p.nq + qb] = own.n_listed;
 }
 
+// Whether the Q blocks are counted once, by kernels of their own, instead of by every CTA that comes after them. What the
+// CTAs do together is half the square of the blocks, times the spans (and about four spans' worth for the rest), times the
+// slices of the heads, at 1.2 span visits a nanosecond; the two kernels cost 5 to 8 us. Without : with them, us, at 8
+// heads: 8 x 8K tokens and 16 spans (2.6e6 visits) 10 : 15, 16 x 8K, 6 (5e6) 12 : 15, 16 x 8K, 16 (10e6) 19 : 17, 4 x 32K,
+// 16, at 32 heads (10e6, counted under the writes) 22 : 30, 32 x 8K, 16 (42e6) 45 : 19, 16 x 32K, 60 (537e6) 425 : 57.
+constexpr double kCountVisits = 16e6;
+bool count_first(long long blocks, int M, int slices) {
+  return 0.5 * static_cast<double>(blocks) * static_cast<double>(blocks) * (M + 4.0) * slices > kCountVisits;
+}
+
 }  // namespace
 }  // namespace omni
 
@@ -227,6 +276,13 @@ extern "C" int omni_attn_build_mask_sm100(const int32_t* modality_positions, int
   if (slices > H) slices = H;
   p.heads_per_cta = (H + slices - 1) / slices;
   const dim3 grid(nq, B, (H + p.heads_per_cta - 1) / p.heads_per_cta);
+  p.counts = p.bases = nullptr;
+  if (count_first(blocks, M, static_cast<int>(grid.z))) {
+    p.counts = static_cast<int32_t*>(scratch);
+    p.bases = p.counts + blocks;
+    mask_count_kernel<<<static_cast<unsigned>((blocks + kMaskThreads - 1) / kMaskThreads), kMaskThreads, 0, st>>>(p);
+    mask_scan_kernel<<<1, kScanThreads, 0, st>>>(p);
+  }
   mask_build_kernel<<<grid, kMaskThreads, 0, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? OMNI_OK : OMNI_ERR_CUDA;
 }

@@ -73,6 +73,27 @@ def test_mask_builder_at_block_edges(cuda_device, n):
                        cpu.partial_block_masks[cpu.partial_block_mask_indices[sel].long()])
 
 
+@pytest.mark.parametrize("B,n,M", [(40, 8190, 8), (1300, 200, 2), (5000, 100, 3)])
+def test_mask_builder_on_thousands_of_blocks(cuda_device, B, n, M):
+    """Batches whose Q blocks are counted by kernels of their own (thousands of them, of 64, two and one for each batch
+    element): lists, types, tiles and their order of the CPU builder."""
+    g = torch.Generator().manual_seed(B)
+    mp = torch.zeros(B, M, 3, dtype=torch.int32)
+    mp[:, :, 1] = torch.randint(0, n + 50, (B, M), generator=g)
+    mp[:, :, 2] = torch.randint(0, 400, (B, M), generator=g)
+    cpu = build_mask(mp, B, 2, n, n)
+    gpu = build_mask(mp.to(cuda_device), B, 2, n, n, device=cuda_device)
+    for name in ("kv_num_blocks", "kv_indices", "block_mask_types"):
+        assert torch.equal(getattr(gpu, name).cpu(), getattr(cpu, name)), name
+    gi = gpu.partial_block_mask_indices.cpu()
+    sel = gi[:, 0] >= 0
+    assert torch.equal(gi >= 0, cpu.partial_block_mask_indices >= 0) and torch.equal(gi[:, 0], gi[:, 1])
+    assert torch.equal(gi[:, 0][sel], torch.arange(int(sel.sum()), dtype=torch.int32))   # numbered in order, none twice
+    assert gpu.partial_block_masks.shape == cpu.partial_block_masks.shape
+    want = cpu.partial_block_masks[cpu.partial_block_mask_indices[:, 0][sel].long()]
+    assert torch.equal(gpu.partial_block_masks[gi[:, 0][sel].long().to(cuda_device)].cpu(), want)
+
+
 @pytest.mark.parametrize("n", [200, 383])
 def test_views_that_start_at_any_element(cuda_device, n):
     """A length that is no multiple of the block may come as a view at any element offset (the rows are copied
