@@ -409,6 +409,7 @@ struct DeviceMask : torch::CustomClassHolder {
   void order_after_build(const at::cuda::CUDAStream& stream) {
     if (stream.stream() != built_on) ready.block(stream);
   }
+  void order_after_build() { order_after_build(at::cuda::getCurrentCUDAStream(device)); }
   const int32_t* partial_idx_ptr() const { return pidx.defined() ? pidx.data_ptr<int32_t>() : nullptr; }
   const uint8_t* partial_bool_ptr() const {
     return pbool.defined() && pbool.numel() > 0 ? reinterpret_cast<const uint8_t*>(pbool.data_ptr<bool>()) : nullptr;
@@ -603,7 +604,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                              std::optional<torch::Tensor> pbool, std::optional<torch::Tensor> pbits, int num_partial,
                              int block, int padded) {
         return c10::make_intrusive<DeviceMask>(nb, idx, types, pidx, pbool, pbits, num_partial, block, padded);
-      }));
+      }))
+      .def("order_after_build", pybind11::overload_cast<>(&DeviceMask::order_after_build),
+           "makes the current stream wait until the mask's tensors are there, and for nothing behind them");
   m.def("operator_forward", &operator_forward, "the operator's forward on a DeviceMask");
   m.def("operator_autograd", &operator_autograd, "the operator's differentiable forward on a DeviceMask");
   m.def("build_mask", &build_mask, "block mask of an interleaved sequence, built on the GPU");

@@ -153,14 +153,11 @@ def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, s
         _check(res)
     mask, nb, idx, typ, pidx, bits, count = res
     device = nb.device
-    built_on = torch.cuda.current_stream(device)
     bm = OmniBlockMask(nb, idx, typ, padded, padded, 128, 128, pidx, None)
 
     def expand_pool() -> Tensor:
         # first read of the reference-shaped pool: waits for the GPU to learn how many tiles there are
-        cur = torch.cuda.current_stream(device)
-        if cur != built_on:
-            cur.wait_stream(built_on)
+        mask.order_after_build()
         need = int(count.item())
         shifts = torch.arange(32, dtype=torch.int32, device=device)
         return ((bits[:need].unsqueeze(-1) >> shifts) & 1).bool().view(need, 128, 128)
@@ -170,7 +167,7 @@ def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, s
     # what omni_attention_forward_out uses; a caller that asks for the byte-per-element pool
     # (pack_bits=False) gets it through the container's field, expanded then
     bm._cache[(str(device), True)] = {"nb": nb, "idx": idx, "typ": typ, "pidx": pidx, "pbool": None, "pbits": bits,
-                                      "num_partial": int(bits.shape[0]), "ready": None, "built_on": built_on}
+                                      "num_partial": int(bits.shape[0]), "order_after_build": mask.order_after_build}
     return bm
 
 
@@ -181,9 +178,7 @@ def _device_mask(bm: OmniBlockMask, device: torch.device, pack_bits: bool) -> di
     if hit is not None:
         # The copies and the pack kernel were enqueued on the stream that was current when the entry
         # was built; a call on another stream must not run ahead of them.
-        cur = torch.cuda.current_stream(device)
-        if cur != hit["built_on"]:
-            cur.wait_event(hit["ready"]) if hit["ready"] is not None else cur.wait_stream(hit["built_on"])
+        hit["order_after_build"]()
         return hit
     cv = lambda t: t.to(device=device, dtype=torch.int32).contiguous()
     d = {"nb": cv(bm.kv_num_blocks), "idx": cv(bm.kv_indices), "typ": cv(bm.block_mask_types),
@@ -198,9 +193,15 @@ def _device_mask(bm: OmniBlockMask, device: torch.device, pack_bits: bool) -> di
             else:
                 d["pbool"] = pool
     with torch.cuda.device(device):
-        d["ready"] = torch.cuda.Event()
-        d["ready"].record(torch.cuda.current_stream(device))
-        d["built_on"] = torch.cuda.current_stream(device)
+        built_on, ready = torch.cuda.current_stream(device), torch.cuda.Event()
+        ready.record(built_on)
+
+    def order_after_build():
+        cur = torch.cuda.current_stream(device)
+        if cur != built_on:
+            cur.wait_event(ready)
+
+    d["order_after_build"] = order_after_build
     bm._cache[key] = d
     return d
 

@@ -114,6 +114,32 @@ def test_views_that_start_at_any_element(cuda_device, n):
         assert torch.equal(a, b)
 
 
+def test_a_call_waits_for_the_mask_and_not_for_later_work_of_its_stream(cuda_device):
+    """A mask built on a side stream that goes on to other work: calls on another stream, and the first read of the byte
+    pool, wait until the mask is there, but do not wait for that work."""
+    n = 256
+    mp = torch.tensor([[[0, 10, 50], [0, 100, 90]]], dtype=torch.int32, device=cuda_device)
+    q = torch.randn(1, 2, n, 64, device=cuda_device).half()
+    first = build_mask(mp, 1, 2, n, n, device=cuda_device)
+    want, pool = omni_attention(q, q, q, first), first.partial_block_masks
+    forward = torch.empty_like(q)
+    omni_attention_forward_out(q, q, q, forward, first, n)   # whatever is set up once is set up
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        bm = build_mask(mp, 1, 2, n, n, device=cuda_device)
+        torch.cuda._sleep(400_000_000)   # about 0.2 s
+        late = side.record_event()
+    out = torch.empty_like(q)
+    omni_attention_forward_out(q, q, q, out, bm, n)
+    same = omni_attention(q, q, q, bm)
+    got = bm.partial_block_masks
+    torch.cuda.current_stream().synchronize()
+    assert not late.query()
+    assert torch.equal(out, want) and torch.equal(same, want) and torch.equal(got, pool)
+    torch.cuda.synchronize()
+
+
 def test_every_refusal_is_an_omni_attn_error(cuda_device):
     """Unaligned tensors of whole blocks, forward and backward, and lists whose shapes do not fit each other or q."""
     n, numel = 256, 2 * 256 * 64
