@@ -70,10 +70,11 @@ struct UnitSlot {
 };
 
 __host__ __device__ constexpr int ws_words_per_block(bool b64) { return b64 ? 4 : 1; }
-__host__ __device__ inline int ws_slot_bytes(int nq, bool b64) {
+// Bytes of one of the two unit slots: a table for each tile of the unit, the schedule, the header.
+__host__ __device__ constexpr int ws_slot_bytes(int nq, bool b64, bool split) {
   const int tab = nq * ws_words_per_block(b64) * 4;
   const int sched = nq * 2;
-  return (2 * tab + sched + 15) / 16 * 16 + static_cast<int>(sizeof(UnitHeader));   // a multiple of 16
+  return ((split ? 1 : 2) * tab + sched + 15) / 16 * 16 + static_cast<int>(sizeof(UnitHeader));   // a multiple of 16
 }
 
 template <int D>
@@ -199,13 +200,13 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   volatile int* abort_flag = misc + 1;
   float* xchg = reinterpret_cast<float*>(after_tiles + Cfg::kBarBytes);   // split form: [2][kXchgCols][128], (max, sum) [2][128]
   uint8_t* slot_base = after_tiles + Cfg::kBarBytes + (SPLIT ? kXchgBytes : 0);
-  const int slot_bytes = ws_slot_bytes(p.nq, B64);
+  const int slot_bytes = ws_slot_bytes(p.nq, B64, SPLIT);
   auto slot = [&](int k) -> UnitSlot {
     uint8_t* b = slot_base + (k & 1) * slot_bytes;
     const int tab_words = p.nq * ws_words_per_block(B64);
     UnitSlot s;
     s.tab[0] = reinterpret_cast<uint32_t*>(b);
-    s.tab[1] = s.tab[0] + tab_words;
+    s.tab[1] = s.tab[0] + (SPLIT ? 0 : tab_words);   // a unit of the split form is one tile
     s.sched = reinterpret_cast<uint16_t*>(s.tab[1] + tab_words);
     s.hdr = reinterpret_cast<UnitHeader*>(b + slot_bytes - sizeof(UnitHeader));
     return s;
@@ -832,8 +833,8 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
 // Dynamic shared memory of one CTA for sequences of nq 128-row tiles.
 template <int D>
-static int ws_smem_bytes(int nq, bool b64, bool split) {
-  return WsCfg<D>::kFixedBytes + 2 * ws_slot_bytes(nq, b64) + (split ? kXchgBytes : 0);
+static constexpr int ws_smem_bytes(int nq, bool b64, bool split) {
+  return WsCfg<D>::kFixedBytes + 2 * ws_slot_bytes(nq, b64, split) + (split ? kXchgBytes : 0);
 }
 
 constexpr int kMaxSmemPerCta = 232448;   // 227 KB, the most one CTA can have on sm_100
@@ -923,9 +924,16 @@ static cudaError_t launch_ws_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
 // the pairs fill the chip: 12 x 4K (1.3) 74 : 72 / 66 : 59 but 32 x 1.5K (1.3) 39 : 47 / 35 : 39, 32 x 2K (1.7) 49 : 64 /
 // 43 : 51. Lists of at most 8 blocks leave too little to halve once the tiles outnumber the SMs: 32 x 1K 31 : 31 / 27 : 27,
 // with images 31 : 33 / 27 : 29.
+// The rule looks at the shape alone, not at the form of the lists: the two forms add a row's blocks up in different
+// orders, and the same mask in 64- and in 128-blocks has to give the same bits. (The last bits of a head do depend on how
+// many heads are computed with it.)
+constexpr int kSplitMaxTiles = 296;   // two for each of 148 SMs, the most that the first condition lets through there
+static_assert(ws_smem_bytes<128>(kSplitMaxTiles, true, true) <= kMaxSmemPerCta &&
+                  ws_smem_bytes<64>(kSplitMaxTiles, true, true) <= kMaxSmemPerCta,
+              "split units fit for every length the rule lets through, in either list form");
 static bool use_split_units(int nq, int BH, int sms) {
   const long long pairs = static_cast<long long>((nq + 1) / 2) * BH, tiles = static_cast<long long>(nq) * BH;
-  return pairs <= sms && (nq > 8 || tiles <= sms);
+  return pairs <= sms && nq <= kSplitMaxTiles && (nq > 8 || tiles <= sms);
 }
 
 template <int D, bool BF16, bool SOFTCAP, bool B64>
@@ -934,8 +942,7 @@ static cudaError_t launch_ws_s(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
   int sms = 0;
   const cudaError_t e = device_sm_count(sms);
   if (e != cudaSuccess) return e;
-  const bool split = use_split_units(p.nq, p.BH, sms) && ws_smem_bytes<D>(p.nq, B64, true) <= kMaxSmemPerCta;
-  return split ? launch_ws_t<D, BF16, SOFTCAP, B64, true>(tmQ, tmK, tmV, p, stream)
+  return use_split_units(p.nq, p.BH, sms) ? launch_ws_t<D, BF16, SOFTCAP, B64, true>(tmQ, tmK, tmV, p, stream)
                : launch_ws_t<D, BF16, SOFTCAP, B64, false>(tmQ, tmK, tmV, p, stream);
 }
 
@@ -955,7 +962,7 @@ static cudaError_t launch_ws_d(const CUtensorMap& tmQ, const CUtensorMap& tmK, c
 int ws_max_tiles(int head_dim, bool b64) {
   const int fixed = head_dim == 128 ? WsCfg<128>::kFixedBytes : WsCfg<64>::kFixedBytes;
   int nq = kMaxKvBlocks;
-  while (nq > 0 && fixed + 2 * ws_slot_bytes(nq, b64) > kMaxSmemPerCta) nq -= 8;
+  while (nq > 0 && fixed + 2 * ws_slot_bytes(nq, b64, false) > kMaxSmemPerCta) nq -= 8;
   return nq;
 }
 

@@ -81,3 +81,19 @@ def test_rows_that_are_zero_whatever_the_inputs_hold(cuda_device, H, D, dtype):
     assert torch.equal(out[:, :, first], want[:, :, first])
     cols = [c for c in range(D) if c != 5]   # 0 * Inf in column 5 of the rows that visit the block
     assert torch.equal(out[:, :, rest][..., cols], want[:, :, rest][..., cols])
+
+
+@pytest.mark.parametrize("H,nq", [(1, 240), (1, 296), (1, 297), (2, 148), (3, 100)])
+def test_long_lists_in_both_block_sizes(cuda_device, H, nq):
+    """Few heads of long sequences, up to and past the most tiles that take the split form: the same mask in 64- and in
+    128-blocks has the same bits at head_dim 128, where the tables of 64-blocks are what fills shared memory."""
+    n = nq * 128 - 70
+    g = torch.Generator(device=cuda_device).manual_seed(nq)
+    q, k, v = (torch.randn(1, H, n, 128, generator=g, device=cuda_device).mul_(0.5).bfloat16() for _ in range(3))
+    masks = [create_causal_omni_block_mask(1, H, n, n, block, block, cuda_device) for block in (128, 64)]
+    (a, la), (b, lb) = (omni_attention(q, k, v, m, return_lse=True) for m in masks)
+    assert torch.equal(a, b) and torch.equal(la, lb)
+    rows = torch.tensor([0, 1, 127, 128, n // 2, n - 1], device=cuda_device)   # a few rows in fp32
+    s = q[:, :, rows].float() @ k.float().transpose(-1, -2) / 128 ** 0.5
+    s = s.masked_fill(torch.arange(n, device=cuda_device) > rows[:, None], float("-inf"))
+    assert_parity(a[:, :, rows], la[:, :, rows], s.softmax(-1) @ v.float(), s.logsumexp(-1), f"{H} x {nq}")
