@@ -280,7 +280,7 @@ int omni_attn_build_mask_sm100(const int32_t* modality_positions, int B, int M, 
  * The list, pool, size, dtype, scale, stream and status arguments are those of omni_attn_fwd_sm100.
  * head_dim 32, 64 or 128 as in the forward; the backward takes 128x128 blocks only (OMNI_ERR_BLOCK_SIZE for
  * 64x64: re-express such a mask on 128-tiles first, as the Python operator does).
- * Three kernels are enqueued on cuda_stream; the result is deterministic (no atomics). */
+ * Two kernels are enqueued on cuda_stream; the result is deterministic (no atomics). */
 long long omni_attn_bwd_workspace_bytes(int B, int H, int seqlen_padded);
 int omni_attn_bwd_sm100(const void* q, const void* k, const void* v, const void* o, const float* lse,
                         const void* d_o, void* dq, void* dk, void* dv, const int32_t* kv_num_blocks,

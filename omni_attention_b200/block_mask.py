@@ -397,24 +397,6 @@ def _limits_from_modality_tensor(modality_positions: Tensor, seq_len: int, padde
     return limits, plain
 
 
-def count_partial_tiles(limits: Tensor, plain: Tensor, block: int = 128) -> int:
-    """Number of PARTIAL tiles of the row-limit mask ``limits`` [B, N] (the same typing rule as
-    ``block_mask_from_row_limits`` and the GPU builder, evaluated from the smallest and largest limit
-    of every block of rows; the pool is shared by the heads)."""
-    B, N = limits.shape
-    nq = N // block
-    lim = limits.long().view(B, nq, block)
-    lim_min, lim_max = lim.min(-1).values, lim.max(-1).values
-    q = torch.arange(N, device=limits.device).view(1, nq, block)
-    causal_block = (plain.view(B, nq, block) & (lim == q)).all(-1)
-    lo = torch.div(lim_min + 1, block, rounding_mode="floor")   # first KV block that is not FULL
-    hi = torch.div(lim_max, block, rounding_mode="floor")       # last KV block that is listed
-    cnt = (hi - lo + 1).clamp(min=0)
-    qb = torch.arange(nq, device=limits.device).view(1, nq)
-    cnt = cnt - ((lo <= qb) & (qb <= hi) & causal_block).long()  # a CAUSAL diagonal tile is not PARTIAL
-    return int(cnt.sum().item())
-
-
 def create_omni_block_mask_from_modality_positions(modality_positions: Tensor, batch: int, nheads: int, q_len: int,
                                                    kv_len: int, Q_BLOCK_SIZE: int = 128, KV_BLOCK_SIZE: int = 128,
                                                    device="cpu") -> OmniBlockMask:

@@ -23,8 +23,8 @@
 // S and dP are recomputed in both kinds (7 tile contractions per visited tile instead of 5), which
 // buys a deterministic result with no atomics and no fp32 dQ buffer.
 // Both are warp-specialised: 8 compute warps (a tile row = TMEM lane is shared by two
-// threads, one per warpgroup, each taking 64 of its 128 columns), one warp whose first lane issues
-// every tcgen05.mma and one whose first lane issues the TMA loads; everything is handed over through
+// threads, one per warpgroup, each taking 64 of its 128 columns), one warp of which an elected lane issues
+// every tcgen05.mma and one of which an elected lane issues the TMA loads; everything is handed over through
 // mbarriers (tcgen05.commit for "MMAs done", thread arrivals for "P / dS stored"). The per-element
 // work of a visit is split in two (probabilities from S; dS from dP and the probabilities) and the
 // MMAs of consecutive visits are interleaved so that the tensor pipe runs under both halves.
@@ -171,20 +171,8 @@ __device__ __forceinline__ void bwd_mma_ss(uint32_t d_tmem, uint32_t sA, uint32_
   }
 }
 
-// acc[128 x D] (+)= A[128 x 128] * B[128 x D], A 16-bit in TMEM (lane = row of A), B a row-major
-// tile whose rows are the contraction index (MN-major operand).
-template <int D>
-__device__ __forceinline__ void bwd_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t sB, uint32_t idesc,
-                                           bool accumulate) {
-  const uint32_t b_lo = umma_desc_lo(sB, BwdCfg<D>::kChunkBytes);
-  umma_ts_lo(d_tmem, a_tmem, b_lo, kBwdDescHi, idesc, accumulate ? 1u : 0u);
-#pragma unroll
-  for (int k = 1; k < kBlock / 16; ++k) {
-    umma_ts_lo_acc(d_tmem, a_tmem + 8 * k, b_lo + k * 128, kBwdDescHi, idesc);
-  }
-}
-
-// The same with the 16-bit A operand stored as two runs of 32 TMEM columns, 64 columns apart
+// acc[128 x D] (+)= A[128 x 128] * B[128 x D], A 16-bit in TMEM (lane = row of A), B a row-major tile whose rows
+// are the contraction index (MN-major operand). A is stored as two runs of 32 TMEM columns, 64 columns apart
 // (contraction indices [0,64) at a_region + a_off, [64,128) at a_region + 64 + a_off): the layout the
 // tile kernels use so that each thread writes P / dS only over score columns it has read itself.
 template <int D>
@@ -292,8 +280,8 @@ __device__ __forceinline__ float lse_to_log2(float lse) {
 // 2. dK, dV. One CTA per (KV block, batch*head), see bwd_decode_cta. 320 threads:
 //   warps 0-7  per-element work; threads t and t + 128 own key row t of the block (query columns
 //              [0,64) and [64,128) of the visited Q block)
-//   warp  8    first lane issues every tcgen05.mma
-//   warp  9    first lane issues the TMA loads
+//   warp  8    an elected lane issues every tcgen05.mma
+//   warp  9    an elected lane issues the TMA loads (at D = 64 all lanes stage LSE and delta)
 // TMEM, D = 128: S^T [0,128), dP^T [128,256), dV [256,384), dK [384,512); P^T (16-bit) goes over S^T and
 // dS^T over dP^T. D = 64: two regions of S^T [0,256), dP^T [256,384), dV [384,448), dK [448,512); P^T and dS^T
 // both go over S^T. Each thread writes only columns it has read itself.

@@ -53,7 +53,7 @@ struct FwdParams {
   float cap_in;          // soft-cap: scale / softcap (0 = no soft-cap)
   float cap_out;         // soft-cap: softcap / scale
   int group_heads;       // heads per scheduling group of the warp-specialised kernel (>= 1)
-  int num_units;         // work units of the warp-specialised kernel: ceil(nq / 2) * BH
+  int num_units;         // work units of the warp-specialised kernel: ceil(nq / 2) * BH pairs of tiles, or nq * BH tiles
   int o_aligned32;       // output base address is 32-byte aligned (256-bit stores allowed)
   int d_real;            // head_dim of the tensors in memory: 32, 64 or 128 (32 is computed as 64 with the
                          // missing columns read as zeros by the TMA unit); row pitch of o is d_real * 2 bytes

@@ -142,9 +142,8 @@ def pack_partial_masks(partial_block_masks: Tensor) -> Tensor:
 def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, seq_len: int, padded: int,
                           device: torch.device) -> OmniBlockMask:
     """Runs omni_attn_build_mask_sm100 on ``device`` and wraps its outputs in an OmniBlockMask whose
-    tensors stay on the device. Nothing here waits for the GPU when ``modality_positions`` is a host
-    tensor: the number of PARTIAL tiles, which sizes the pool, is counted on the host from the span
-    table (O(B*N*M) integer arithmetic). The kernels write the pool bit-packed, which is what the
+    tensors stay on the device. Nothing here waits for the GPU: the pool of PARTIAL tiles is sized by what a
+    sequence of that many blocks can need at most. The kernel writes the pool bit-packed, which is what the
     attention kernels read; the container's byte-per-element ``partial_block_masks`` is expanded from it
     only if somebody reads that field."""
     res = load_extension().build_mask(modality_positions, batch, nheads, int(seq_len), int(padded),
@@ -159,6 +158,8 @@ def build_block_mask_cuda(modality_positions: Tensor, batch: int, nheads: int, s
         # first read of the reference-shaped pool: waits for the GPU to learn how many tiles there are
         mask.order_after_build()
         need = int(count.item())
+        if need > bits.shape[0]:
+            raise OmniAttnError(f"mask builder: {need} PARTIAL tiles in a pool of {bits.shape[0]}")
         shifts = torch.arange(32, dtype=torch.int32, device=device)
         return ((bits[:need].unsqueeze(-1) >> shifts) & 1).bool().view(need, 128, 128)
 
