@@ -536,8 +536,9 @@ __device__ __forceinline__ void bwd_dkdv_cta(const CUtensorMap& tmQ, const CUten
     const float2 c2 = make_float2(p.f.scale_log2, p.f.scale_log2);
     int next_qb = n_vis > 0 ? vis_s[0] : 0;   // looked up one visit ahead
     uint32_t next_code = code_s[next_qb];
-    for (int i = 0; i < n_vis; ++i) {
-      const int stage = i % Cfg::kQStages;
+    int turn = 0;   // i % 3, counted: divided, it is a register too many in the soft-capped kernel (112 bytes of spills, 32 now)
+    for (int i = 0; i < n_vis; ++i, turn = turn == 2 ? 0 : turn + 1) {
+      const int stage = Cfg::kAhead ? turn : i & 1;
       const uint32_t ph = static_cast<uint32_t>(i & 1);
       const int qb = next_qb;
       const uint32_t code = next_code;
