@@ -424,7 +424,7 @@ omni_fwd_ws_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int j = 0; j < kXchgCols / 2; ++j) {
             const float a = f_mine * __uint_as_float(own[2 * j]) + f_other * x_other[(2 * j) * kBlock];
             const float b = f_mine * __uint_as_float(own[2 * j + 1]) + f_other * x_other[(2 * j + 1) * kBlock];
-            w[j] = pack2<BF16>(empty ? 0.f : a, empty ? 0.f : b);
+            w[j] = empty ? 0u : pack2<BF16>(a, b);
           }
           mbar_arrive(bar_xfree + 8 * (g ^ 1));
           if (have_row && col < p.d_real) {
