@@ -296,7 +296,7 @@ __device__ __forceinline__ float lse_to_log2(float lse) {
 // half of the per-element work waits for more than the pair in front of it. (With the regions alternating,
 // S^T(i+1) over dP^T(i) and so only after E2(i), the chain S^T - E1 - E2 of a visit could not overlap the next
 // one's: kernel 1055 against 949 us for 32 heads x 8K tokens at D = 128, bits equal.) The 32 MMAs of a visit are
-// then 2 560 of its about 3 000 cycles (80 each: their operands and the TMA writes share the shared-memory port).
+// 2 048 of its about 3 000 cycles; both kinds of CTA together keep the tensor pipe busy for 66 % of the active cycles.
 // D = 64 needs half the MMAs and is bound by the per-element work; its second region of S^T lets the scores run a
 // visit ahead, so that E1(i+1) starts as soon as E2(i) ends:
 //   dV(i) | dP^T(i+1), dK(i), S^T(i+2)
