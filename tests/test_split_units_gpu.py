@@ -16,8 +16,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("D,dtype", [(32, torch.float16), (64, torch.bfloat16), (128, torch.bfloat16), (128, torch.float16)])
 @pytest.mark.parametrize("H,nq,rest", [(1, 1, 0), (2, 2, 5), (3, 5, 63), (1, 9, 1), (38, 8, 0)])
 def test_lists_of_any_length(cuda_device, H, nq, rest, D, dtype, block, softcap):
-    """Against the oracle with the tolerance of the parity contract. 38 heads of 8 tiles are 304 units, two or
-    three for each SM. `rest` tokens are missing from the last block."""
+    """Against the oracle with the tolerance of the parity contract. 38 heads of 8 tiles are just past the rule
+    and run as pairs (split units that outnumber the SMs: test_long_lists_in_both_block_sizes). `rest` tokens are missing from the last block."""
     g = torch.Generator().manual_seed(100 * nq + D)
     padded = nq * 128
     bm = random_fcp_block_mask(1, H, padded, seed=nq, block=block)
